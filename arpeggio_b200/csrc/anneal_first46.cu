@@ -1,0 +1,8 @@
+// First accept on compressed dDI problems, four and six copies, integer fields: the kernels of anneal_group.cuh.
+#include "anneal_group.cuh"
+
+namespace arp {
+cudaError_t int_first46(const DDParams& a, int P, int warps, cudaStream_t st) {
+  return P == 4 ? grp::dispatch<4, grp::kFirst>(a, warps, st) : grp::dispatch<6, grp::kFirst>(a, warps, st);
+}
+}  // namespace arp

@@ -92,6 +92,19 @@ struct ReadParams {
   float* llr = nullptr;       // (B, D * nb), positive = bit 1
 };
 
+// Integer anneals (anneal_group.cuh), one file per rule and copy count; Philox round keys filled in, warps 0: by
+// occupancy, else the block width.
+cudaError_t int_first2(const DDParams& a, int warps, cudaStream_t st);
+cudaError_t int_first46(const DDParams& a, int P, int warps, cudaStream_t st);
+cudaError_t int_warm(const DDParams& a, int warps, cudaStream_t st);
+cudaError_t int_chord2(const DDParams& a, int warps, cudaStream_t st);
+cudaError_t int_chord46(const DDParams& a, int P, int warps, cudaStream_t st);
+cudaError_t int_engine(const DDParams& a, int P, cudaStream_t st);
+int tuned_warps(int NS, int P, int policy, int precision);
+// Host-side checks shared by the anneal entry points.
+int check_dd(const void* Gt, const void* h, const void* T, int L, int P, int R, int D, int B, const uint32_t* inst,
+             int start, const int8_t* out_s, const void* out_de, const int64_t* out_st);
+
 // policy: 0 first accept, 1 Chord round; flt: FP32 fields.  Shapes already validated.
 cudaError_t anneal_dispatch(int policy, bool flt, const DDParams& a, int P, int warps, cudaStream_t st);
 cudaError_t map_dispatch(const MapParams& a, cudaStream_t st);

@@ -222,8 +222,8 @@ int arp_soft_trajectory(const float* J, const float* hf, const float* h0, const 
                         const uint32_t* inst, uint32_t k0, uint32_t k1, float* m0, float* m1, float* best_d,
                         int8_t* best_l, void* stream);
 
-/* Autotuner hook (no reference counterpart): warps per block (1, 2, 4 or 8; 0 restores the occupancy heuristic)
- * of the compressed-problem anneal kernels for problems of D coordinates (by 32-wide slot count), P copies,
+/* Autotuner hook (no reference counterpart): warps per block (1, 2, 4 or 8; 0 restores the occupancy heuristic; a
+ * warp holds one to eight anneals) of the compressed-problem anneal kernels for problems of D coordinates (by 32-wide slot count), P copies,
  * policy (0 first accept, 1 Chord round, 2 the warm-started first accept of arp_anneal_first_accept_warm*, P = 2
  * and int32 only) and precision (0 int32, 1 FP32 fields).  Process-wide; results do not depend on it (anneals are
  * independent of their block). */

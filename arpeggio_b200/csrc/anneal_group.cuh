@@ -628,11 +628,11 @@ struct Widths {
 };
 constexpr size_t kMaxDynamic = 226 * 1024;
 
-template <int LN, int C, int P, Rule RULE, int MB = min_blocks<LN, C>()>
-static cudaError_t launch(const DDParams& a, int warps, cudaStream_t st) {
-  constexpr int A = 32 / LN, WMAX = max_threads<LN, C>() / 32;
-  const auto kern = k_anneal_grp<LN, C, P, RULE, MB>;
-  static Widths wd;
+// Launches kern for the A anneals per warp and blocks of at most WMAX warps it was compiled for; smem(W): its dynamic
+// shared memory with blocks of W warps, key: a number that differs where smem does.
+template <int A, int WMAX, typename Kern, typename Smem>
+static cudaError_t launch_widths(Widths& wd, Kern kern, size_t key, Smem smem, const DDParams& a, int warps,
+                                 cudaStream_t st) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
@@ -643,19 +643,18 @@ static cudaError_t launch(const DDParams& a, int warps, cudaStream_t st) {
     d.limit = bytes;
     return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   };
-  const size_t key = sched_bytes<P>(a.L) + 1;
-  if (d.key != key) {
+  if (d.key != key + 1) {
     if ((e = cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
     const size_t was = d.limit;
     if ((e = limit(kMaxDynamic)) != cudaSuccess) return e;
     for (int i = 0; i < 5; ++i) {
       d.nb[i] = 0;
-      const size_t s = smem_bytes<LN, C, P>(a.L, 1 << i);
-      if ((1 << i) > WMAX || s > kMaxDynamic) continue;
-      if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.nb[i], kern, 32 << i, s)) != cudaSuccess) return e;
+      if ((1 << i) > WMAX || smem(1 << i) > kMaxDynamic) continue;
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.nb[i], kern, 32 << i, smem(1 << i));
+      if (e != cudaSuccess) return e;
     }
     if ((e = limit(was)) != cudaSuccess) return e;
-    d.key = key;
+    d.key = key + 1;
   }
   const int(&nb)[5] = d.nb;
   const int sms = d.sms;
@@ -669,7 +668,7 @@ static cudaError_t launch(const DDParams& a, int warps, cudaStream_t st) {
   while (wi > 0 && (1 << (wi - 1)) * A >= a.R) --wi;
   // one anneal per warp: blocks of four warps while every block finds an SM of its own (one 32-user frame: 44 us
   // against 46 with eight; 64 frames: 69 against 63)
-  if (LN == 32 && warps <= 0 && wi == 3 && (long long)a.B * ((a.R + 3) / 4) <= sms) wi = 2;
+  if (A == 1 && warps <= 0 && wi == 3 && (long long)a.B * ((a.R + 3) / 4) <= sms) wi = 2;
   if (nb[wi] == 0) return cudaErrorInvalidConfiguration;
   const int W = 1 << wi;
   // small batches: each problem's anneals over several blocks, so that the batch still fills the GPU
@@ -678,9 +677,16 @@ static cudaError_t launch(const DDParams& a, int warps, cudaStream_t st) {
   const int most = (a.R + W * A - 1) / (W * A);
   long long sp = a.B < slots ? (slots + a.B - 1) / a.B : 1;
   b.split = (int)(sp < most ? sp : most);
-  const size_t smem = smem_bytes<LN, C, P>(a.L, W);
-  if (smem > d.limit && (e = limit(smem)) != cudaSuccess) return e;
-  return launch_ex(kern, dim3((unsigned)((long long)a.B * b.split)), dim3(W * 32), smem, st, a.B <= kPdlMaxB, b);
+  if (smem(W) > d.limit && (e = limit(smem(W))) != cudaSuccess) return e;
+  return launch_ex(kern, dim3((unsigned)((long long)a.B * b.split)), dim3(W * 32), smem(W), st, a.B <= kPdlMaxB, b);
+}
+
+template <int LN, int C, int P, Rule RULE, int MB = min_blocks<LN, C>()>
+static cudaError_t launch(const DDParams& a, int warps, cudaStream_t st) {
+  static Widths wd;
+  return launch_widths<32 / LN, max_threads<LN, C>() / 32>(
+      wd, k_anneal_grp<LN, C, P, RULE, MB>, sched_bytes<P>(a.L), [&](int W) { return smem_bytes<LN, C, P>(a.L, W); }, a,
+      warps, st);
 }
 
 // Warps of a call up to which one anneal per warp is the faster mapping: what the unbounded kernels (about 100

@@ -100,6 +100,9 @@ cudaError_t int_warm(const DDParams& a, int warps, cudaStream_t st);
 cudaError_t int_chord2(const DDParams& a, int warps, cudaStream_t st);
 cudaError_t int_chord46(const DDParams& a, int P, int warps, cudaStream_t st);
 cudaError_t int_engine(const DDParams& a, int P, cudaStream_t st);
+// FP32-field anneals (anneal_group_f32.cuh), one file per rule.
+cudaError_t f32_first(const DDParams& a, int P, int warps, cudaStream_t st);
+cudaError_t f32_chord(const DDParams& a, int P, int warps, cudaStream_t st);
 int tuned_warps(int NS, int P, int policy, int precision);
 // Host-side checks shared by the anneal entry points.
 int check_dd(const void* Gt, const void* h, const void* T, int L, int P, int R, int D, int B, const uint32_t* inst,

@@ -1,4 +1,4 @@
-"""Integer anneals with several anneals per warp, bit for bit against the oracle: coordinate counts at the edges of
+"""Anneals with several anneals per warp, bit for bit against the oracle: coordinate counts at the edges of
 every lanes x coordinates mapping, anneal counts that leave groups of a warp idle, batches on both sides of the
 dispatch's anneal counts, and schedules and coefficients on both sides of the 32-bit energies' range."""
 import os
@@ -56,6 +56,28 @@ def test_every_mapping_equals_the_oracle(D, P, policy):
     c = rng.integers(-200, 200, len(T)) if policy == 'chord' else None
     _check(D, P, 3, 5, T, 60, 'bal', policy, c)
     _check(D, P, 126, 33, T[:5 * P - 1], 60, 'rand', policy, None if c is None else c[:5 * P - 1])
+
+
+@pytest.mark.parametrize('policy', ['arpeggio', 'chord'])
+@pytest.mark.parametrize('D,P', SHAPES)
+def test_every_float_mapping_equals_the_oracle(D, P, policy):
+    """The FP32 rule is one rounding per operation in a fixed order, so every mapping gives the oracle's bits."""
+    from arpeggio_b200 import arpeggiofx
+    rng = np.random.default_rng(D * 8 + P)
+    T = rng.uniform(0.02, 0.3, 7 * P - 1).astype(np.float32)
+    c = rng.uniform(-0.1, 0.1, len(T)).astype(np.float32) if policy == 'chord' else None
+    for B, R, start in ((3, 5, 'bal'), (126, 33, 'rand')):
+        G, h = (x.astype(np.float32) / np.float32(4096) for x in _problems(D, B, 3))
+        inst, key = np.arange(B, dtype=np.int64) + 5, 0x77 + (0x1234 << 32)
+        ref = O.anneal_dd_f32(G, h, P, R, T, 0.02, inst, key, start, policy, c, nthreads=NTH)
+        dev = lambda x: torch.from_numpy(np.ascontiguousarray(x)).cuda()
+        s, de, st, status = arpeggiofx.anneal(dev(G.transpose(0, 2, 1)), dev(h), P, R, dev(T), 0.02,
+                                              dev(inst.astype(np.int32)), key, start, policy,
+                                              None if c is None else dev(c), 'f32')
+        torch.cuda.synchronize()
+        assert int(status.item()) == 0
+        for got, want in zip((s, de, st), ref):
+            assert np.array_equal(got.cpu().numpy(), want)
 
 
 def test_two_and_four_anneals_per_warp_at_64_coordinates():

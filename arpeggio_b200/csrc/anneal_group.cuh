@@ -376,11 +376,16 @@ __device__ __forceinline__ void run(const DDParams& a, const PhiloxKeys& K, cons
               const int32_t s4 = (sm & -8) ^ 4;
               const bool sn = (snap >> c) & 1u;
               int jl = 32;
-              for (;;) {
-                const bool acc = sn && lane < jl;
-                const uint32_t m = __ballot_sync(ARP_FULL, acc);
-                if (m == 0) break;
-                commit(c, acc, m, s4, (w[c] ^ sm) - sm + dg[c] - 1, jl);  // psi = s w + 2 G_jj
+              if constexpr (LN == 32) {  // one anneal: its flips are the ballot's bits
+                for (uint32_t m = __ballot_sync(ARP_FULL, sn); m != 0; m &= (1u << jl) - 1u)
+                  commit(c, true, m, s4, (w[c] ^ sm) - sm + dg[c] - 1, jl);  // psi = s w + 2 G_jj
+              } else {
+                for (;;) {
+                  const bool acc = sn && lane < jl;
+                  const uint32_t m = __ballot_sync(ARP_FULL, acc);
+                  if (m == 0) break;
+                  commit(c, acc, m, s4, (w[c] ^ sm) - sm + dg[c] - 1, jl);
+                }
               }
             }
             if (a.out_n1) n1 += (__ballot_sync(ARP_FULL, (fb >> (p * C)) != 0) & gmask) != 0;

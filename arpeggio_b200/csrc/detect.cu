@@ -100,105 +100,163 @@ __device__ __forceinline__ float row_dot(const float (&x)[TB], const float (&y)[
   return hsum16(v);
 }
 
-// The D x D work is tiled over a GS x GS (16 x 16) thread grid: thread (ty, tx) owns rows ty*TB .. ty*TB+TB-1
-// and columns tx*TB .. tx*TB+TB-1 of Q and of the inverse, in registers.  Dp = GS TB >= D; padded rows and
-// columns of H are zero and the padded diagonal of A is 1, so the inverse's D x D block is unchanged.  (A 32 x 32
-// grid of 2 x 2 tiles was measured for one frame and is slower: the 64 elimination steps are latency-bound and
-// a 1024-thread barrier per step costs more than the smaller tiles save.)
+// The D x D work is tiled over 16 columns of threads (tx) by TY rows (ty) per use: a thread owns rows ty RB ..
+// ty RB + RB - 1 and columns tx TB .. tx TB + TB - 1 of Q and of the inverse, in registers, pairs of rows packed for
+// the two-wide FP32 multiply-add (the same roundings).  Dp = 16 TB >= D; padded rows and columns of H are zero and the
+// padded diagonal of A is 1, so the inverse's D x D block is unchanged.  A block holds U uses (U Dp = 64 rows of one
+// MMA for Dp <= 64).  What bounds the map is issue slots and the elimination's latency (one barrier a step), so:
+//   tall tiles: an elimination step loads RB + TB values and forms RB factors for RB TB multiply-adds.  8 x 4 on
+//     128 threads (37 k instructions per 32-user use, then the code's own fetches) against 4 x 4 on 256 (45 k, the
+//     previous kernel): 16384 32-user uses 0.90 -> 0.76 ms; a batch of 444 uses or fewer keeps 4 x 4;
+//   several uses per block where D is small, which share the barriers and the MMAs: 49999 8-user uses 1.04 -> 0.35 ms,
+//     16384 16-user ones 0.42 -> 0.27;
+//   little code: what one thread per row or one loop can do (levels, outputs) is not unrolled over the tile.
 // Gram on the tensor cores: digit planes of one row chunk (CH rows of H) in the canonical K-major no-swizzle
-// layout of 8-bit operands -- core matrices of 8 rows (coordinates) x 16 bytes (rows of H), LBO = 128 B between
-// neighbours along K, SBO = (CH / 16) 128 B between 8-coordinate groups; one MMA consumes K = 32 (two core
-// matrices).  MP = the MMA's M: 64 for Dp <= 64 (rows Dp .. 63 zero), else 128.
+// layout of 8-bit operands -- core matrices of 8 rows (coordinates, the uses' one after another) x 16 bytes (rows of
+// H), LBO = 128 B between neighbours along K, SBO = (CH / 16) 128 B between 8-coordinate groups; one MMA consumes K = 32
+// (two core matrices).  MP = the MMA's M and N: 64 for Dp <= 64, else 128; with several uses the blocks off the
+// diagonal are computed and ignored.
 template <int Dp>
 __host__ __device__ constexpr int kMmaM() { return Dp <= 64 ? 64 : 128; }
 template <int Dp>
 __host__ __device__ constexpr int kPlaneBytes() { return kMmaM<Dp>() * kChunkRows<Dp>(); }
-template <int Dp>
-__host__ __device__ constexpr int kTmemCols() {  // four class accumulators of Dp columns, a power of two >= 32
-  return 4 * Dp <= 32 ? 32 : (4 * Dp <= 64 ? 64 : (4 * Dp <= 128 ? 128 : (4 * Dp <= 256 ? 256 : 512)));
-}
 
 // The digit pairs (a, b) of each class a + b = 6, 5, 4, 3, in issue order.
 __constant__ int8_t kPairA[10] = {3, 3, 2, 3, 1, 2, 3, 0, 2, 1};
 __constant__ int8_t kPairB[10] = {3, 2, 3, 1, 3, 2, 0, 3, 1, 2};
 __constant__ int8_t kPairC[10] = {0, 1, 1, 2, 2, 2, 3, 3, 3, 3};  // accumulator: class 6 - c
 
-// Register bounds for more resident blocks (the Gauss-Jordan steps are barrier-latency bound, so blocks overlap):
-// four per SM at 32 users (64 registers, a few spilled: 3.95 -> 3.73 ms per 65536 uses), two per SM at 64 users
-// (126 registers: 28.8 -> 19.3 ms per 65536 uses); the same outputs bit for bit.
-template <int TB, int GS>
-__global__ void __launch_bounds__(GS * GS, TB == 8 ? 2 : (TB == 4 ? 4 : 1)) k_map_dd(const MapParams a) {
-  constexpr int Dp = GS * TB, QP = Dp + 4, NT = GS * GS;
-  constexpr int CH = kChunkRows<Dp>(), MP = kMmaM<Dp>(), KG = CH / 16, PB = kPlaneBytes<Dp>();
-  constexpr uint32_t NCOL = kTmemCols<Dp>();
+// Two FP32 values in one 64-bit register: per element the same rounding as the scalar operation.
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+// Shape of the map for TB columns and RB_ rows per thread and U_ uses per block.
+template <int TB, int RB_, int U_>
+struct MapShape {
+  static constexpr int Dp = 16 * TB, U = U_, RB = RB_, TPU = 16 * (Dp / RB);
+  static constexpr int NT = U * TPU, HP = Dp + 4, QP = Dp + 4, CH = kChunkRows<Dp>(), MP = kMmaM<Dp>();
+  static constexpr int PB = kPlaneBytes<Dp>(), WPU = TPU / 32;  // bytes of a digit plane, warps per use
+  static constexpr uint32_t NCOL = 4 * MP;                      // four class accumulators
+  static constexpr int kFront = PB > U * Dp * QP ? PB : U * Dp * QP;  // floats: four digit planes, later Q
+  // resident blocks the registers are bounded for: 96 a thread at 64 coordinates, 128 at 128
+  static constexpr int MB = TB == 8 ? 2 : TB == 4 && RB == 8 ? 5 : 3;
+  static constexpr size_t smem() {
+    return sizeof(float) * (kFront + U * (CH * HP + 6 * Dp + CH) + NT / 32);
+  }
+};
+
+template <int TB, int RB_, int U_>
+__global__ void __launch_bounds__(MapShape<TB, RB_, U_>::NT, MapShape<TB, RB_, U_>::MB) k_map_dd(const MapParams a) {
+  using S = MapShape<TB, RB_, U_>;
+  constexpr int Dp = S::Dp, U = S::U, RB = S::RB, TPU = S::TPU, NT = S::NT, HP = S::HP, QP = S::QP, CH = S::CH;
+  constexpr int MP = S::MP, KG = CH / 16, PB = S::PB, WPU = S::WPU, NP = RB / 2;
+  constexpr uint32_t NCOL = S::NCOL;
   extern __shared__ __align__(128) float smap[];
-  uint8_t* planes = reinterpret_cast<uint8_t*>(smap);  // 4 digit planes, PB bytes each (aliases Qs below)
-  float* Hc = smap + (PB * 4 > Dp * QP * 4 ? PB : Dp * QP);  // CH x Dp
-  float* Qs = smap;                            // Dp x QP, written once the Gram's MMAs have completed
-  float* rk = Hc + CH * Dp;       // 2 x Dp (double-buffered row k)
-  float* ck = rk + 2 * Dp;        // 2 x Dp (double-buffered column k)
-  float* gv = ck + 2 * Dp;        // Dp
-  float* xv = gv + Dp;            // Dp
-  float* red = xv + Dp;           // NT / 32
-  float* yc = red + NT / 32;      // CH: the chunk's rows of y
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int us = tid / TPU, ut = tid - us * TPU, tx = ut & 15, ty = ut >> 4;
+  uint8_t* planes = reinterpret_cast<uint8_t*>(smap);  // 4 digit planes, PB bytes each (aliases Q below)
+  float* Hall = smap + S::kFront;                      // U x CH x HP
+  float* Hc = Hall + us * CH * HP;
+  float* Qs = smap + us * Dp * QP;                     // Dp x QP, written once the Gram's MMAs have completed
+  float* rk = Hall + U * CH * HP + us * 6 * Dp;  // 2 x Dp (double-buffered row k)
+  float* ck = rk + 2 * Dp;                       // 2 x Dp (double-buffered column k)
+  float* gv = ck + 2 * Dp;                       // Dp
+  float* xv = gv + Dp;                           // Dp
+  float* yc = Hall + U * (CH * HP + 6 * Dp) + us * CH;  // CH: the chunk's rows of y
+  float* red = Hall + U * (CH * HP + 6 * Dp + CH);      // NT / 32
   __shared__ __align__(8) uint64_t mma_bar;
   __shared__ uint32_t s_tmem;
-  __shared__ int s_abort, s_exp;
-  const int D = a.D, NR2 = a.NR2, b = blockIdx.x;
-  const int tid = threadIdx.x, tx = tid % GS, ty = tid / GS, lane = tid & 31, warp = tid >> 5;
+  __shared__ int s_abort, s_exp[U];
+  const int D = a.D, NR2 = a.NR2;
+  const int b = blockIdx.x * U + us;
+  const bool on = U == 1 || b < a.B;  // the last block may hold fewer uses: the others stage zeros and write nothing
   if (tid == 0) {
     umma::mbar_init(&mma_bar, 1);
     umma::fence_mbar_init();
     s_abort = 0;
   }
-  const int u = a.idx ? a.idx[b] : b;
+  const int u = on ? (a.idx ? a.idx[b] : b) : 0;
   const float* Hb = a.H + (size_t)u * NR2 * D;
   const float* yb = a.y + (size_t)u * NR2;
   // ---- the use's power-of-two scale (largest |H| just below 2^30 after scaling): from the staged rows when they
   //      fit one chunk, else from a pass over H first
   const bool one_chunk = NR2 <= CH;
-  auto set_scale = [&](float mx) {  // mx: this thread's part; every thread leaves with s_exp set
+  auto use_max = [&](float v) {  // the maximum over the use's threads, in all of them (two barriers of the block)
 #pragma unroll
-    for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(ARP_FULL, mx, o));
-    if (lane == 0) red[warp] = mx;
+    for (int o = 16; o; o >>= 1) v = fmaxf(v, __shfl_xor_sync(ARP_FULL, v, o));
+    if (lane == 0) red[warp] = v;
     __syncthreads();
-    if (tid == 0) {
-      float m = 0.0f;
-      for (int w = 0; w < NT / 32; ++w) m = fmaxf(m, red[w]);
+    float m = 0.0f;
+#pragma unroll
+    for (int w = 0; w < WPU; ++w) m = fmaxf(m, red[us * WPU + w]);
+    return m;
+  };
+  auto set_scale = [&](float mx) {  // every thread leaves with s_exp set
+    const float m = use_max(mx);
+    if (ut == 0) {
       int e = 0;
       if (m > 0.0f) frexpf(m, &e);  // m in [2^(e-1), 2^e)
-      s_exp = m > 0.0f ? 30 - e : 0;
+      s_exp[us] = m > 0.0f ? 30 - e : 0;
     }
     __syncthreads();
   };
   if (!one_chunk) {
     float mx = 0.0f;
-    for (int x = tid; x < NR2 * D; x += NT) mx = fmaxf(mx, fabsf(Hb[x]));
+    if (on) {
+      const int n4 = (reinterpret_cast<uintptr_t>(Hb) & 15u) == 0 ? NR2 * D / 4 : 0;
+#pragma unroll 8
+      for (int x = ut; x < n4; x += TPU) {
+        const float4 v = reinterpret_cast<const float4*>(Hb)[x];
+        mx = fmaxf(fmaxf(mx, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
+      }
+#pragma unroll 4
+      for (int x = 4 * n4 + ut; x < NR2 * D; x += TPU) mx = fmaxf(mx, fabsf(Hb[x]));
+    }
     set_scale(mx);
   }
   float gacc = 0.0f;
-  constexpr uint32_t IDESC = umma::idesc_s8(MP, Dp);
+  constexpr uint32_t IDESC = umma::idesc_s8(MP, MP);
   const uint32_t pbase = umma::su32(planes);
   int nchunk = 0;
   for (int r0 = 0; r0 < NR2; r0 += CH, ++nchunk) {
     const int nr = min(CH, NR2 - r0);
     __syncthreads();  // the previous chunk's digits were read by MMAs that have completed (waited below)
     if (s_abort) break;
-    for (int x = tid; x < nr; x += NT) yc[x] = yb[r0 + x];
+    for (int x = ut; x < nr; x += TPU) yc[x] = on ? yb[r0 + x] : 0.0f;
     float mx = 0.0f;
-    if (D == Dp && (D & 3) == 0) {
-      const float4* src = reinterpret_cast<const float4*>(Hb + (size_t)r0 * D);
-      float4* dst = reinterpret_cast<float4*>(Hc);
-      for (int x = tid; x < nr * Dp / 4; x += NT) {
-        const float4 v = src[x];
-        dst[x] = v;
+    if ((D & 3) == 0 && (reinterpret_cast<uintptr_t>(a.H) & 15u) == 0) {  // 16-byte loads, Dp / 4 threads a row
+      constexpr int QR = Dp / 4, RS = TPU / QR;
+      const int q4 = 4 * (ut & (QR - 1));
+      const bool in = on && q4 < D;
+#pragma unroll 4
+      for (int r = ut / QR; r < nr; r += RS) {
+        const float4 v = in ? *reinterpret_cast<const float4*>(Hb + (size_t)(r0 + r) * D + q4)
+                            : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        *reinterpret_cast<float4*>(Hc + r * HP + q4) = v;
         mx = fmaxf(fmaxf(mx, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
       }
     } else {
-      for (int x = tid; x < nr * Dp; x += NT) {
+#pragma unroll 2
+      for (int x = ut; x < nr * Dp; x += TPU) {
         const int r = x / Dp, j = x - r * Dp;
-        const float v = j < D ? Hb[(size_t)(r0 + r) * D + j] : 0.0f;
-        Hc[x] = v;
+        const float v = on && j < D ? Hb[(size_t)(r0 + r) * D + j] : 0.0f;
+        Hc[r * HP + j] = v;
         mx = fmaxf(mx, fabsf(v));
       }
     }
@@ -206,26 +264,29 @@ __global__ void __launch_bounds__(GS * GS, TB == 8 ? 2 : (TB == 4 ? 4 : 1)) k_ma
       set_scale(mx);  // its barriers also publish the staged rows
     else
       __syncthreads();
-    const int sx = s_exp;
-    if (tid < Dp)
-      for (int r = 0; r < nr; ++r) gacc = __fmaf_rn(Hc[r * Dp + tid], yc[r], gacc);
+    if (ut < Dp)
+      for (int r = 0; r < nr; ++r) gacc = __fmaf_rn(Hc[r * HP + ut], yc[r], gacc);
     // digit planes: a warp writes one core matrix (8 coordinates x 16 rows) at a time, lane = coordinate m % 8
-    // + 8 (row quad), one 32-bit word of four rows per plane (conflict-free); rows >= nr and coordinates >= Dp
-    // are zero.  The signed digits of x (|x| < 2^30) are the bytes of (x + 0x808080) ^ 0x808080: adding 128 at each
-    // of the three low digit positions makes every low byte u_a = d_a + 128 with the borrow carried up, and the
-    // XOR turns u_a into d_a's two's-complement byte; the top byte is d3.  A 4 x 4 byte transpose (eight byte
-    // permutes) turns four rows' digit words into one word per plane.
+    // + 8 (row quad), one 32-bit word of four rows per plane (conflict-free); rows >= nr are zero.  The signed digits
+    // of x (|x| < 2^30) are the bytes of (x + 0x808080) ^ 0x808080: adding 128 at each of the three low digit positions
+    // makes every low byte u_a = d_a + 128 with the borrow carried up, and the XOR turns u_a into d_a's two's-complement
+    // byte; the top byte is d3.  A 4 x 4 byte transpose (eight byte permutes) turns four rows' digit words into one
+    // word per plane.
     const int ksteps = (nr + 31) >> 5;
-    const bool fast_scale = sx >= -126 && sx <= 127;
-    const float fs = fast_scale ? __int_as_float((sx + 127) << 23) : 1.0f;
-    for (int cm = warp; cm < (MP / 8) * KG; cm += NT / 32) {
-      const int mg = cm / KG, kg = cm - mg * KG;
+    constexpr int NG = U * Dp / 8;  // rows of the MMA beyond the uses' coordinates stay as they are, their results unused
+    for (int cm = warp; cm < NG * 2 * ksteps; cm += NT / 32) {
+      const int kg = cm / NG, mg = cm - kg * NG;
       const int m = mg * 8 + (lane & 7), k0 = kg * 16 + (lane >> 3) * 4;
+      const int mu = m / Dp, mj = m - mu * Dp;
+      const float* hc = Hall + mu * CH * HP + mj;
+      const int sx = s_exp[mu];
+      const bool fast_scale = sx >= -126 && sx <= 127;
+      const float fs = fast_scale ? __int_as_float((sx + 127) << 23) : 1.0f;
       uint32_t z[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int k = k0 + i;
-        const float v = (m < Dp && k < nr) ? Hc[k * Dp + m] : 0.0f;
+        const float v = k < nr ? hc[k * HP] : 0.0f;
         const int32_t x = __float2int_rn(fast_scale ? __fmul_rn(v, fs) : ldexpf(v, sx));
         z[i] = ((uint32_t)x + 0x808080u) ^ 0x808080u;
       }
@@ -254,7 +315,7 @@ __global__ void __launch_bounds__(GS * GS, TB == 8 ? 2 : (TB == 4 ? 4 : 1)) k_ma
           const uint64_t bd = umma::sdesc(pbase + kPairB[q] * PB + ks * 256, 128, KG * 128);
           // the first product of each class in the first chunk starts its accumulator
           const bool first = nchunk == 0 && ks == 0 && (q == 0 || q == 1 || q == 3 || q == 6);
-          umma::mma_s8(tmem + (uint32_t)(kPairC[q] * Dp), ad, bd, IDESC, first ? 0u : 1u);
+          umma::mma_s8(tmem + (uint32_t)(kPairC[q] * MP), ad, bd, IDESC, first ? 0u : 1u);
         }
       }
       umma::commit(&mma_bar);
@@ -275,34 +336,38 @@ __global__ void __launch_bounds__(GS * GS, TB == 8 ? 2 : (TB == 4 ? 4 : 1)) k_ma
   }
   // ---- epilogue: each entry of Q from the four class accumulators, summed exactly as an integer
   //      P = ((c6 2^8 + c5) 2^8 + c4) 2^8 + c3 (|P| < 2^50), converted once with rounding to nearest and scaled by
-  //      2^(24 - 2s) (exact).  TMEM lane of row m: m (M = 128), or m % 16 + 32 (m / 16) (M = 64); warps w and w + 4
-  //      read lanes 32 (w % 4) .. + 31, the first and the second half of the columns.
+  //      2^(24 - 2s) (exact).  TMEM lane of row m: m (M = 128), or m % 16 + 32 (m / 16) (M = 64); a warp reads lanes
+  //      32 (w % 4) .. + 31, of one use's rows, and its share of that use's columns.
   {
-    const int wq = warp & 3, half = warp >> 2;
-    const int m = MP == 128 ? wq * 32 + lane : wq * 16 + lane;
-    const bool valid = (MP == 128 || lane < 16) && m < Dp;
-    const int e2 = 24 - 2 * s_exp;
+    constexpr int RQ = MP / 4, NH = NT / 128, CW = Dp >= 8 * NH ? Dp / NH : 8;  // rows per quarter, column shares
+    const int wq = warp & 3, share = warp >> 2;
+    const bool used = U * Dp >= MP || wq * RQ < U * Dp;  // (a warp's whole quarter)
+    const int eu = used ? wq * RQ / Dp : 0, m = wq * RQ + lane - eu * Dp;
+    const bool valid = used && lane < RQ;
+    float* Qe = smap + eu * Dp * QP;
+    const int e2 = 24 - 2 * s_exp[eu];
     // scaling by 2^e2 as one multiply where 2^e2 is a normal float (the same correctly rounded product as ldexpf)
     const bool fast_e2 = e2 >= -126 && e2 <= 127;
     const float f2 = fast_e2 ? __int_as_float((e2 + 127) << 23) : 1.0f;
-    constexpr int CW = Dp >= 16 ? Dp / 2 : Dp;
 #pragma unroll 1
-    for (int c0 = half * CW; c0 < (half + 1) * CW && c0 < Dp; c0 += 8) {
+    for (int c0 = share * CW; c0 < (share + 1) * CW && c0 < Dp; c0 += 8) {
       uint32_t v6[8], v5[8], v4[8], v3[8];
-      const uint32_t ta = tmem + ((uint32_t)(wq * 32) << 16) + (uint32_t)c0;
+      const uint32_t ta = tmem + ((uint32_t)(wq * 32) << 16) + (uint32_t)(eu * Dp + c0);
       umma::tmem_ld8_nowait(ta, v6);
-      umma::tmem_ld8_nowait(ta + Dp, v5);
-      umma::tmem_ld8_nowait(ta + 2 * Dp, v4);
-      umma::tmem_ld8_nowait(ta + 3 * Dp, v3);
+      umma::tmem_ld8_nowait(ta + MP, v5);
+      umma::tmem_ld8_nowait(ta + 2 * MP, v4);
+      umma::tmem_ld8_nowait(ta + 3 * MP, v3);
       umma::tmem_wait_ld();
       if (valid) {
+        float qv[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const long long q = ((((long long)(int32_t)v6[j] * 256 + (int32_t)v5[j]) * 256 + (int32_t)v4[j]) * 256) +
                               (int32_t)v3[j];
           const float qf = __ll2float_rn(q);
-          Qs[m * QP + c0 + j] = fast_e2 ? __fmul_rn(qf, f2) : ldexpf(qf, e2);
+          qv[j] = fast_e2 ? __fmul_rn(qf, f2) : ldexpf(qf, e2);
         }
+        sts_vec<8>(Qe + m * QP + c0, qv);
       }
     }
   }
@@ -310,92 +375,127 @@ __global__ void __launch_bounds__(GS * GS, TB == 8 ? 2 : (TB == 4 ? 4 : 1)) k_ma
   __syncthreads();
   if (warp == 0) umma::tmem_free(tmem, NCOL);
   pdl_trigger();  // the chain's next kernel may launch and set up; it waits for this grid before reading
-  float A[TB][TB];
+  uint64_t A[NP][TB];  // rows 2 i, 2 i + 1 of the tile side by side
   float qmax = 0.0f;
-  const float s2 = a.xg ? 0.0f : a.sigma2[b];  // only the MMSE solve reads sigma2 (null for a given guess)
+  const float s2 = a.xg || !on ? 0.0f : a.sigma2[b];  // only the MMSE solve reads sigma2 (null for a given guess)
 #pragma unroll
-  for (int i = 0; i < TB; ++i) lds_vec<TB>(Qs + (ty * TB + i) * QP + tx * TB, A[i]);  // TB floats per access
+  for (int i = 0; i < NP; ++i) {
+    float q[2][TB];
 #pragma unroll
-  for (int i = 0; i < TB; ++i)
+    for (int h = 0; h < 2; ++h) {
+      lds_vec<TB>(Qs + (ty * RB + 2 * i + h) * QP + tx * TB, q[h]);
 #pragma unroll
-    for (int j = 0; j < TB; ++j) {
-      const int gi = ty * TB + i, gj = tx * TB + j;
-      qmax = fmaxf(qmax, fabsf(A[i][j]));
-      if (gi == gj) A[i][j] = gi < D ? __fadd_rn(A[i][j], s2) : 1.0f;
+      for (int j = 0; j < TB; ++j) {
+        const int gi = ty * RB + 2 * i + h, gj = tx * TB + j;
+        qmax = fmaxf(qmax, fabsf(q[h][j]));
+        if (gi == gj) q[h][j] = gi < D ? __fadd_rn(q[h][j], s2) : 1.0f;
+      }
     }
-  if (tid < Dp) gv[tid] = gacc;
+#pragma unroll
+    for (int j = 0; j < TB; ++j) A[i][j] = pack2(q[0][j], q[1][j]);
+  }
+  if (ut < Dp) gv[ut] = gacc;
   if (a.xg) {
     // the guess is given (MDI stages): map around it, no MMSE solve
-    if (tid < Dp) {
-      const float lv = tid < D ? (float)a.xg[(size_t)u * a.xg_stride + tid] : 0.0f;
-      xv[tid] = lv;
-      if (tid < D) a.xq[(size_t)b * D + tid] = (int8_t)lv;
+    if (ut < Dp) {
+      const float lv = on && ut < D ? (float)a.xg[(size_t)u * a.xg_stride + ut] : 0.0f;
+      xv[ut] = lv;
+      if (on && ut < D) a.xq[(size_t)b * D + ut] = (int8_t)lv;
     }
     __syncthreads();
   } else {
     // ---- in-place Gauss-Jordan inverse of A = Q + sigma2 I (SPD, no pivoting), one barrier per step;
-    //      k = kt*TB + kr with kr unrolled so the register tile is always indexed at compile time
-    for (int kt = 0; kt < GS; ++kt) {
+    //      k = kt*RB + kr with kr unrolled so the register tile is always indexed at compile time
+    for (int kt = 0; kt < Dp / RB; ++kt) {
 #pragma unroll
-      for (int kr = 0; kr < TB; ++kr) {
-        const int k = kt * TB + kr, buf = (k & 1) * Dp;
+      for (int kr = 0; kr < RB; ++kr) {
+        const int k = kt * RB + kr, buf = (k & 1) * Dp;
+        const int kc = kr % TB;                              // the step's column in its owners' tiles
+        const bool colown = tx == kt * (RB / TB) + kr / TB;  // (RB is a multiple of TB)
         if (ty == kt) {
-          float rw[TB];
+          float rw[TB], t;
 #pragma unroll
-          for (int j = 0; j < TB; ++j) rw[j] = A[kr][j];
+          for (int j = 0; j < TB; ++j) {
+            if (kr & 1)
+              unpack2(A[kr / 2][j], t, rw[j]);
+            else
+              unpack2(A[kr / 2][j], rw[j], t);
+          }
           sts_vec<TB>(rk + buf + tx * TB, rw);
         }
-        if (tx == kt) {
-          float cw[TB];
+        if (colown) {
 #pragma unroll
-          for (int i = 0; i < TB; ++i) cw[i] = A[i][kr];
-          sts_vec<TB>(ck + buf + ty * TB, cw);
+          for (int i = 0; i < NP; ++i) reinterpret_cast<uint64_t*>(ck + buf + ty * RB)[i] = A[i][kc];
         }
         __syncthreads();
         const float inv = __frcp_rn(rk[buf + k]);
-        float f[TB], rj[TB];
-        lds_vec<TB>(ck + buf + ty * TB, f);
+        const uint64_t ninv = pack2(-inv, -inv);
+        float rj[TB];
         lds_vec<TB>(rk + buf + tx * TB, rj);
+        uint64_t nf[NP], rd[TB];  // minus the factors of the row pairs; the pivot row's entries twice
+        {
+          float f[RB];
+          lds_vec<RB>(ck + buf + ty * RB, f);
 #pragma unroll
-        for (int i = 0; i < TB; ++i) f[i] = __fmul_rn(f[i], inv);
+          for (int i = 0; i < NP; ++i) nf[i] = mul2(pack2(f[2 * i], f[2 * i + 1]), ninv);
+        }
 #pragma unroll
-        for (int i = 0; i < TB; ++i)
+        for (int j = 0; j < TB; ++j) rd[j] = pack2(rj[j], rj[j]);
 #pragma unroll
-          for (int j = 0; j < TB; ++j) A[i][j] = __fmaf_rn(-f[i], rj[j], A[i][j]);
+        for (int i = 0; i < NP; ++i)
+#pragma unroll
+          for (int j = 0; j < TB; ++j) A[i][j] = fma2(nf[i], rd[j], A[i][j]);
+        auto set = [&](uint64_t& v, float x) {  // the pair's half of row kr
+          float lo, hi;
+          unpack2(v, lo, hi);
+          v = (kr & 1) ? pack2(lo, x) : pack2(x, hi);
+        };
         if (ty == kt) {
 #pragma unroll
-          for (int j = 0; j < TB; ++j) A[kr][j] = __fmul_rn(rj[j], inv);
+          for (int j = 0; j < TB; ++j) set(A[kr / 2][j], __fmul_rn(rj[j], inv));
         }
-        if (tx == kt) {
+        if (colown) {
 #pragma unroll
-          for (int i = 0; i < TB; ++i) A[i][kr] = -f[i];
-          if (ty == kt) A[kr][kr] = inv;
+          for (int i = 0; i < NP; ++i) A[i][kc] = nf[i];
+          if (ty == kt) set(A[kr / 2][kc], inv);
         }
       }
     }
     // ---- z = A^-1 g, mu = diag(A^-1 Q) (Q symmetric: sum_j Ainv_ij Q_ij), x_q
-    float zp[TB], mp[TB], gj[TB];
+    float zp[RB], mp[RB], gj[TB];
     lds_vec<TB>(gv + tx * TB, gj);
 #pragma unroll
-    for (int i = 0; i < TB; ++i) {
-      float ar[TB], qj[TB];
-      lds_vec<TB>(Qs + (ty * TB + i) * QP + tx * TB, qj);
+    for (int i = 0; i < RB; ++i) {
+      float ar[TB], qj[TB], t;
+      lds_vec<TB>(Qs + (ty * RB + i) * QP + tx * TB, qj);
 #pragma unroll
-      for (int j = 0; j < TB; ++j) ar[j] = A[i][j];
+      for (int j = 0; j < TB; ++j) {
+        if (i & 1)
+          unpack2(A[i / 2][j], t, ar[j]);
+        else
+          unpack2(A[i / 2][j], ar[j], t);
+      }
       zp[i] = row_dot<TB>(ar, gj);
       mp[i] = row_dot<TB>(ar, qj);
     }
-    if (tx == 0) {
+    if (tx == 0) {  // to shared memory (row buffer: the last step's readers of its halves are behind a barrier)
 #pragma unroll
-      for (int i = 0; i < TB; ++i) {
-        const int gi = ty * TB + i;
-        const float zu = gi < D ? __fdiv_rn(zp[i], mp[i]) : 0.0f;
-        const float lv = gi < D ? nearest_level(zu, a.M) : 0.0f;
-        xv[gi] = lv;
-        if (gi < D) a.xq[(size_t)b * D + gi] = (int8_t)lv;
-        if (a.zs && gi < D) a.zs[(size_t)b * D + gi] = zu;
-        ck[gi] = gi < D ? nearest_level(zp[i], a.M) : 0.0f;  // RI map: spins of the unbiased z (mimo.py:148)
+      for (int i = 0; i < RB; ++i) {
+        xv[ty * RB + i] = zp[i];
+        ck[Dp + ty * RB + i] = mp[i];
       }
+    }
+    __syncthreads();
+    if (ut < Dp) {
+      const float z = xv[ut];
+      const float zu = ut < D ? __fdiv_rn(z, ck[Dp + ut]) : 0.0f;
+      const float lv = ut < D ? nearest_level(zu, a.M) : 0.0f;
+      if (on && ut < D) {
+        a.xq[(size_t)b * D + ut] = (int8_t)lv;
+        if (a.zs) a.zs[(size_t)b * D + ut] = zu;
+      }
+      ck[ut] = ut < D ? nearest_level(z, a.M) : 0.0f;  // RI map: spins of the unbiased z (mimo.py:148)
+      xv[ut] = lv;
     }
     __syncthreads();
   }
@@ -405,10 +505,10 @@ __global__ void __launch_bounds__(GS * GS, TB == 8 ? 2 : (TB == 4 ? 4 : 1)) k_ma
     const int N = qam ? 2 * D : D;
     float off = 0.0f, dgm = 0.0f, gm = 0.0f;
 #pragma unroll
-    for (int i = 0; i < TB; ++i)
+    for (int i = 0; i < RB; ++i)
 #pragma unroll
       for (int j = 0; j < TB; ++j) {
-        const int gi = ty * TB + i, gj = tx * TB + j;
+        const int gi = ty * RB + i, gj = tx * TB + j;
         if (gi < D && gj < D) {
           const float v = fabsf(Qs[gi * QP + gj]);
           if (gi == gj)
@@ -417,23 +517,17 @@ __global__ void __launch_bounds__(GS * GS, TB == 8 ? 2 : (TB == 4 ? 4 : 1)) k_ma
             off = fmaxf(off, v);
         }
       }
-    if (tid < D) gm = fabsf(gv[tid]);
-    float sc = qam ? fmaxf(fmaxf(4.0f * off, 2.0f * dgm), 4.0f * gm) : fmaxf(off, 2.0f * gm);
-#pragma unroll
-    for (int o = 16; o; o >>= 1) sc = fmaxf(sc, __shfl_xor_sync(ARP_FULL, sc, o));
-    if (lane == 0) red[tid >> 5] = sc;
-    __syncthreads();
-    sc = 0.0f;
-#pragma unroll
-    for (int w = 0; w < NT / 32; ++w) sc = fmaxf(sc, red[w]);
-    sc = fmaxf(sc, 1e-12f);
-    if (tid == 0) a.scale[b] = sc;
+    if (ut < D) gm = fabsf(gv[ut]);
+    const float sc =
+        fmaxf(use_max(qam ? fmaxf(fmaxf(4.0f * off, 2.0f * dgm), 4.0f * gm) : fmaxf(off, 2.0f * gm)), 1e-12f);
+    if (!on) return;
+    if (ut == 0) a.scale[b] = sc;
     float* Jo = a.Jri + (size_t)b * N * N;
 #pragma unroll
-    for (int i = 0; i < TB; ++i)
+    for (int i = 0; i < RB; ++i)
 #pragma unroll
       for (int j = 0; j < TB; ++j) {
-        const int gi = ty * TB + i, gj = tx * TB + j;
+        const int gi = ty * RB + i, gj = tx * TB + j;
         if (gi >= D || gj >= D) continue;
         const float q = Qs[gi * QP + gj];
         if (qam) {
@@ -446,7 +540,7 @@ __global__ void __launch_bounds__(GS * GS, TB == 8 ? 2 : (TB == 4 ? 4 : 1)) k_ma
         }
       }
     const float r2 = __fmul_rn(2.0f, a.r_reg);
-    for (int i = tid; i < D; i += NT) {
+    for (int i = ut; i < D; i += TPU) {
       const float lv = ck[i];
       const float hv[2] = {qam ? __fmul_rn(4.0f, gv[i]) : __fmul_rn(2.0f, gv[i]), __fmul_rn(2.0f, gv[i])};
       const float sp[2] = {qam ? (lv > 0.0f ? 1.0f : -1.0f) : lv, (lv == 3.0f || lv == -1.0f) ? 1.0f : -1.0f};
@@ -461,66 +555,61 @@ __global__ void __launch_bounds__(GS * GS, TB == 8 ? 2 : (TB == 4 ? 4 : 1)) k_ma
     return;
   }
   // ---- h = 2 (g - Q x_q), scale = max(|h|, |Q|)
-  float hp[TB], xj[TB];
+  float hp[RB], xj[TB];
   lds_vec<TB>(xv + tx * TB, xj);
 #pragma unroll
-  for (int i = 0; i < TB; ++i) {
+  for (int i = 0; i < RB; ++i) {
     float qj[TB];
-    lds_vec<TB>(Qs + (ty * TB + i) * QP + tx * TB, qj);
+    lds_vec<TB>(Qs + (ty * RB + i) * QP + tx * TB, qj);
     hp[i] = row_dot<TB>(qj, xj);
-    hp[i] = __fmul_rn(2.0f, __fsub_rn(gv[ty * TB + i], hp[i]));
-    if (ty * TB + i < D) qmax = fmaxf(qmax, fabsf(hp[i]));
+    hp[i] = __fmul_rn(2.0f, __fsub_rn(gv[ty * RB + i], hp[i]));
+    if (ty * RB + i < D) qmax = fmaxf(qmax, fabsf(hp[i]));
+    if (tx == 0) ck[ty * RB + i] = hp[i];
   }
-#pragma unroll
-  for (int o = 16; o; o >>= 1) qmax = fmaxf(qmax, __shfl_xor_sync(ARP_FULL, qmax, o));
-  if (lane == 0) red[tid >> 5] = qmax;
-  __syncthreads();
-  float sc = 0.0f;
-#pragma unroll
-  for (int w = 0; w < NT / 32; ++w) sc = fmaxf(sc, red[w]);
-  sc = fmaxf(sc, 1e-12f);
-  if (tid == 0) a.scale[b] = sc;
-  // ---- outputs: G = Q / scale (x 4096, rounded half to even), h likewise
+  const float sc = fmaxf(use_max(qmax), 1e-12f);
+  if (!on) return;
+  if (ut == 0) a.scale[b] = sc;
+  // ---- outputs: G = Q / scale (x 4096, rounded half to even), h likewise; TB columns of a row per thread
   const bool quant = a.qscale > 0.0f;
+  auto out = [&](float q) {  // the entry's 32 bits
+    const float v = __fdiv_rn(q, sc);
+    return quant ? (int32_t)rintf(__fmul_rn(v, a.qscale)) : __float_as_int(v);
+  };
+  int32_t* Go = reinterpret_cast<int32_t*>(a.G) + (size_t)b * D * D;
+  const bool vec = TB >= 4 && (D & 3) == 0 && (reinterpret_cast<uintptr_t>(a.G) & 15u) == 0;
+#pragma unroll 1
+  for (int gi = ty; gi < D; gi += Dp / RB) {
+    float q[TB];
+    lds_vec<TB>(Qs + gi * QP + tx * TB, q);
+    int32_t g[TB];
 #pragma unroll
-  for (int i = 0; i < TB; ++i) {
-    const int gi = ty * TB + i;
-    if (gi >= D) continue;
+    for (int j = 0; j < TB; ++j) g[j] = out(q[j]);
+    int32_t* o = Go + (size_t)gi * D + tx * TB;
+    if constexpr (TB >= 4) {
+      if (vec) {
 #pragma unroll
-    for (int j = 0; j < TB; ++j) {
-      const int gj = tx * TB + j;
-      if (gj >= D) continue;
-      const float v = __fdiv_rn(Qs[gi * QP + gj], sc);
-      if (quant)
-        reinterpret_cast<int32_t*>(a.G)[((size_t)b * D + gi) * D + gj] = (int32_t)rintf(__fmul_rn(v, a.qscale));
-      else
-        reinterpret_cast<float*>(a.G)[((size_t)b * D + gi) * D + gj] = v;
+        for (int j = 0; j < TB; j += 4)
+          if (tx * TB + j < D) *reinterpret_cast<int4*>(o + j) = make_int4(g[j], g[j + 1], g[j + 2], g[j + 3]);
+        continue;
+      }
     }
-    if (tx == 0) {
-      const float v = __fdiv_rn(hp[i], sc);
-      if (quant)
-        reinterpret_cast<int32_t*>(a.h)[(size_t)b * D + gi] = (int32_t)rintf(__fmul_rn(v, a.qscale));
-      else
-        reinterpret_cast<float*>(a.h)[(size_t)b * D + gi] = v;
-    }
+#pragma unroll
+    for (int j = 0; j < TB; ++j)
+      if (tx * TB + j < D) o[j] = g[j];
   }
+  if (ut < D) reinterpret_cast<int32_t*>(a.h)[(size_t)b * D + ut] = out(ck[ut]);
 }
 
-template <int TB, int GS>
-static size_t map_smem() {
-  constexpr int Dp = GS * TB, PB = kPlaneBytes<Dp>();
-  constexpr size_t front = PB * 4 > Dp * (Dp + 4) * 4 ? (size_t)PB : (size_t)Dp * (Dp + 4);  // planes | Qs, floats
-  return sizeof(float) * (front + (size_t)kChunkRows<Dp>() * (Dp + 1) + 6 * (size_t)Dp + GS * GS / 32);
-}
-
-template <int TB, int GS = 16>
+template <int TB, int RB, int U>
 static cudaError_t launch_map(const MapParams& a, cudaStream_t st) {
-  const size_t smem = map_smem<TB, GS>();
+  using S = MapShape<TB, RB, U>;
+  constexpr size_t smem = S::smem();
   if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k_map_dd<TB, GS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e =
+        cudaFuncSetAttribute(k_map_dd<TB, RB, U>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  k_map_dd<TB, GS><<<a.B, GS * GS, smem, st>>>(a);
+  k_map_dd<TB, RB, U><<<(a.B + U - 1) / U, S::NT, smem, st>>>(a);
   return cudaGetLastError();
 }
 
@@ -839,10 +928,17 @@ __global__ void __launch_bounds__(kReadThreads) k_readout_dd(const ReadParams a)
 
 namespace arp {
 
+// Small batches, whose blocks all run at once, take a use per block and low tiles (more threads a use, less serial work
+// each); others the tall tiles, several uses per block up to 32 coordinates.
+constexpr int kMapSmall = 444;
+
 cudaError_t map_dispatch(const MapParams& a, cudaStream_t st) {
   const int D = a.D;
-  return D <= 16 ? launch_map<1>(a, st) : D <= 32 ? launch_map<2>(a, st) : D <= 64 ? launch_map<4>(a, st)
-                                                                          : launch_map<8>(a, st);
+  const bool small = a.B <= kMapSmall;
+  if (D > 64) return launch_map<8, 8, 1>(a, st);
+  if (D > 32) return small ? launch_map<4, 4, 1>(a, st) : launch_map<4, 8, 1>(a, st);
+  if (D > 16) return small ? launch_map<2, 2, 1>(a, st) : launch_map<2, 4, 2>(a, st);
+  return small ? launch_map<1, 2, 1>(a, st) : launch_map<1, 4, 4>(a, st);
 }
 
 static size_t readout_smem(int D, int NR2, int R, bool soft = false) {

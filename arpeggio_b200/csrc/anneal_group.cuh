@@ -225,7 +225,7 @@ __device__ __forceinline__ void run(const DDParams& a, const PhiloxKeys& K, cons
     for (int q4 = 0; k < L; ++q4) {
       if constexpr (!WIDE) {
         // thresholds ceil(u 4T / 2^32) of the quad's four sweeps, 16 bits each, sweeps (0, 1) and (2, 3) in a word
-#pragma unroll(C * P <= 8 ? P : 1)
+#pragma unroll(C * P <= 8 ? P : LN == 32 ? 2 : 1)
         for (int p = 0; p < P; ++p) {
           uint32_t t4[4];
 #pragma unroll
@@ -299,6 +299,8 @@ __device__ __forceinline__ void run(const DDParams& a, const PhiloxKeys& K, cons
               return (int32_t)hi;
             }
           };
+          // whether the pass may have flipped (known for free with one anneal per warp and in the skipped scan)
+          bool any = LN != 32 || k == 0;
           // one round of slot c: every group with a candidate (acc on some lane of m) flips its first
           auto commit = [&](int c, bool acc, uint32_t m, int32_t s4, int32_t psi, int& jl) {
             const int32_t v = acc ? s4 : 0;
@@ -316,17 +318,19 @@ __device__ __forceinline__ void run(const DDParams& a, const PhiloxKeys& K, cons
               fb |= 1u << (p * C + c);
             }
             jl = l;
+            if constexpr (LN == 32) any = true;
           };
           if constexpr (!CHORD && HOIST) {
-            int32_t x[C], any = 0;
+            int32_t x[C], zs = 0;
 #pragma unroll
             for (int c = 0; c < C; ++c) {
               const int32_t sm = -(int32_t)((dn >> (p * C + c)) & 1u);
               x[c] = (kappa(c) - Bk - dg[c]) ^ ~sm;
               w[c] += x[c];
-              any |= w[c] ^ sm;
+              zs |= w[c] ^ sm;
             }
-            if (__any_sync(ARP_FULL, any < 0)) {
+            any = __any_sync(ARP_FULL, zs < 0) || k == 0;
+            if (any) {
 #pragma unroll
               for (int c = 0; c < C; ++c) {
                 const int32_t sm = -(int32_t)((dn >> (p * C + c)) & 1u);
@@ -390,16 +394,18 @@ __device__ __forceinline__ void run(const DDParams& a, const PhiloxKeys& K, cons
             }
             if (a.out_n1) n1 += (__ballot_sync(ARP_FULL, (fb >> (p * C)) != 0) & gmask) != 0;
           }
-          if constexpr (LN == 32 && !WIDE) {
-            e = __reduce_add_sync(ARP_FULL, e);
-          } else {
+          if (any) {
+            if constexpr (LN == 32 && !WIDE) {
+              e = __reduce_add_sync(ARP_FULL, e);
+            } else {
 #pragma unroll
-            for (int o = LN / 2; o; o >>= 1) e += __shfl_xor_sync(ARP_FULL, e, o);
-          }
-          de += e;
-          if (de < best) {  // best state after each pass (arpeggio_fx.cu:90-93)
-            best = de;
-            bdn = dn ^ fb;
+              for (int o = LN / 2; o; o >>= 1) e += __shfl_xor_sync(ARP_FULL, e, o);
+            }
+            de += e;
+            if (de < best) {  // best state after each pass (arpeggio_fx.cu:90-93)
+              best = de;
+              bdn = dn ^ fb;
+            }
           }
           ++k;
         }
@@ -676,12 +682,20 @@ static cudaError_t launch_widths(Widths& wd, Kern kern, size_t key, Smem smem, c
   if (A == 1 && warps <= 0 && wi == 3 && (long long)a.B * ((a.R + 3) / 4) <= sms) wi = 2;
   if (nb[wi] == 0) return cudaErrorInvalidConfiguration;
   const int W = 1 << wi;
-  // small batches: each problem's anneals over several blocks, so that the batch still fills the GPU
+  // small batches: each problem's anneals over several blocks, as many as make the call shortest in anneals one after
+  // another per warp times waves of blocks (each further block stages the problem once more)
   DDParams b = a;
-  const long long slots = (long long)nb[wi] * sms;
+  b.split = 1;
+  const double slots = (double)nb[wi] * sms;
   const int most = (a.R + W * A - 1) / (W * A);
-  long long sp = a.B < slots ? (slots + a.B - 1) / a.B : 1;
-  b.split = (int)(sp < most ? sp : most);
+  double best = 0.0;
+  for (int s = 1; a.B < 4 * slots && s <= most && s * (long long)a.B < 8 * slots + a.B; ++s) {
+    const double waves = a.B * s / slots, cost = ((a.R + W * A * s - 1) / (W * A * s)) * (waves > 1.0 ? waves : 1.0) + 0.02 * s;
+    if (s == 1 || cost < best) {
+      best = cost;
+      b.split = s;
+    }
+  }
   if (smem(W) > d.limit && (e = limit(smem(W))) != cudaSuccess) return e;
   return launch_ex(kern, dim3((unsigned)((long long)a.B * b.split)), dim3(W * 32), smem(W), st, a.B <= kPdlMaxB, b);
 }
@@ -694,12 +708,15 @@ static cudaError_t launch(const DDParams& a, int warps, cudaStream_t st) {
       warps, st);
 }
 
-// Warps of a call up to which one anneal per warp is the faster mapping: what the unbounded kernels (about 100
-// registers at two coordinates a lane) and the ones bound to 64 registers keep resident at once, 16 and 32 a SM; and
-// anneals up to which two per warp (64 coordinates) beat four, which need four times as many to fill the GPU.  32 users,
-// 32 anneals, one / two / four per warp: 64 uses 63 / 83 / 126 us, 148 uses 121 / 108 / 143, 600 uses
-// 387 / 296 / 308, 1200 uses 727 / 522 / 512.
-constexpr long long kLatWarps = 148LL * 16, kOnePerWarp = 148LL * 32, kTwoPerWarp = 148LL * 32 * 8;
+// How many anneals share a warp is a matter of how many there are: A per warp need A times as many to fill the GPU.
+// Warps of a call up to which one anneal per warp is the fastest: what the unbounded kernels (about 100 registers at two
+// coordinates a lane) and the ones bound to 64 registers keep resident at once, 16 and 32 a SM; then anneals up to
+// which half the full mapping's anneals per warp win, by coordinates.  32 anneals a use, one / two / four per warp at
+// 64 coordinates: 64 uses 63 / 83 / 126 us, 148 uses 121 / 108 / 143, 600 uses 387 / 296 / 308, 1200 uses
+// 727 / 522 / 512; one / two / four at 32: 156 uses 56 / 54 / 63, 312 uses 93 / 75 / 75, 625 uses 184 / 147 / 121;
+// two / four / eight at 16: 156 uses 31 / 35 / 47, 625 uses 84 / 65 / 68, 1250 uses 133 / 106 / 103.
+constexpr long long kLatWarps = 148LL * 16, kOnePerWarp = 148LL * 32;
+constexpr long long kMid16 = 30000, kMid32 = 10000, kMid64 = 148LL * 32 * 8;
 
 // The mapping (LN lanes per anneal, C coordinates per lane) for D coordinates.  P = 6 keeps four coordinates a lane
 // (24 spin bits); the engine's numbers use the same family.
@@ -707,22 +724,29 @@ template <int P, Rule RULE>
 static cudaError_t dispatch(const DDParams& a, int warps, cudaStream_t st) {
   const int D = a.D;
   const long long n = (long long)a.B * a.R, w8 = (long long)a.B * ((a.R + 7) / 8 * 8);
-  if (RULE != kEngine && w8 <= kLatWarps)
+  // (above 64 coordinates an unbounded block fills the SM's registers, half the warps; there, or with few anneals a use,
+  // which would leave two anneals per warp too few warps beside 64 KB of G, one per warp at 128 registers)
+  if constexpr (RULE != kEngine && P < 6)
+    if (D > 64 && w8 > kLatWarps / 2 && (w8 <= kLatWarps || a.R < 16))
+      return D <= 96 ? launch<32, 3, P, RULE>(a, warps, st) : launch<32, 4, P, RULE>(a, warps, st);
+  if (RULE != kEngine && w8 <= (D > 64 ? kLatWarps / 2 : kLatWarps))
     return D <= 32   ? launch<32, 1, P, RULE, 1>(a, warps, st)
            : D <= 64 ? launch<32, 2, P, RULE, 1>(a, warps, st)
            : D <= 96 ? launch<32, 3, P, RULE, 1>(a, warps, st)
                      : launch<32, 4, P, RULE, 1>(a, warps, st);
+  if (RULE != kEngine && w8 <= kOnePerWarp && D <= 64)
+    return D <= 32 ? launch<32, 1, P, RULE>(a, warps, st) : launch<32, 2, P, RULE>(a, warps, st);
+  // few anneals a use leave a wide block's warps without work: the half mapping below 16
+  if (D <= 16 && (n <= kMid16 || a.R < 16)) return launch<8, 2, P, RULE>(a, warps, st);
+  if (D <= 32 && D > 16 && (n <= kMid32 || a.R < 16)) return launch<16, 2, P, RULE>(a, warps, st);
+  if (D <= 16) return launch<4, 4, P, RULE>(a, warps, st);
+  if (D <= 32) return launch<8, 4, P, RULE>(a, warps, st);
   if constexpr (RULE == kEngine || P == 6) {
-    return D <= 16   ? launch<4, 4, P, RULE>(a, warps, st)
-           : D <= 32 ? launch<8, 4, P, RULE>(a, warps, st)
-           : D <= 64 ? launch<16, 4, P, RULE>(a, warps, st)
+    return D <= 64   ? launch<16, 4, P, RULE>(a, warps, st)
+           : D <= 96 ? launch<32, 3, P, RULE>(a, warps, st)
                      : launch<32, 4, P, RULE>(a, warps, st);
   } else {
-    if (w8 <= kOnePerWarp && D <= 64)
-      return D <= 32 ? launch<32, 1, P, RULE>(a, warps, st) : launch<32, 2, P, RULE>(a, warps, st);
-    if (D <= 16) return launch<4, 4, P, RULE>(a, warps, st);
-    if (D <= 32) return launch<8, 4, P, RULE>(a, warps, st);
-    if (D <= 64 && n <= kTwoPerWarp) return launch<16, 4, P, RULE>(a, warps, st);
+    if (D <= 64 && (n <= kMid64 || a.R < 16)) return launch<16, 4, P, RULE>(a, warps, st);
     return D <= 48   ? launch<8, 6, P, RULE>(a, warps, st)
            : D <= 64 ? launch<8, 8, P, RULE>(a, warps, st)
            : D <= 96 ? launch<16, 6, P, RULE>(a, warps, st)

@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(grp::max_threads<LN, C>(), MB) k_anneal_f32(co
     int k = 0;
     for (int q4 = 0; k < L; ++q4) {
       // thresholds of the quad's four sweeps
-#pragma unroll(C * P <= 8 ? P : 1)
+#pragma unroll(C * P <= 8 ? P : LN == 32 ? 2 : 1)
       for (int p = 0; p < P; ++p) {
         float A4[4];
 #pragma unroll
@@ -281,24 +281,30 @@ static cudaError_t launch(const DDParams& a, int warps, cudaStream_t st) {
 template <int P, bool CHORD>
 static cudaError_t dispatch(const DDParams& a, int warps, cudaStream_t st) {
   const int D = a.D;
-  const long long w8 = (long long)a.B * ((a.R + 7) / 8 * 8);
-  if (w8 <= grp::kLatWarps)
+  const long long n = (long long)a.B * a.R, w8 = (long long)a.B * ((a.R + 7) / 8 * 8);
+  if constexpr (P < 6)
+    if (D > 64 && w8 > grp::kLatWarps / 2 && (w8 <= grp::kLatWarps || a.R < 16 || (a.R == 16 && D > 96)))
+      return D <= 96 ? launch<32, 3, P, CHORD>(a, warps, st) : launch<32, 4, P, CHORD>(a, warps, st);
+  if (w8 <= (D > 64 ? grp::kLatWarps / 2 : grp::kLatWarps))
     return D <= 32   ? launch<32, 1, P, CHORD, 1>(a, warps, st)
            : D <= 64 ? launch<32, 2, P, CHORD, 1>(a, warps, st)
            : D <= 96 ? launch<32, 3, P, CHORD, 1>(a, warps, st)
                      : launch<32, 4, P, CHORD, 1>(a, warps, st);
-  if constexpr (P == 6)
-    return D <= 16   ? launch<4, 4, P, CHORD>(a, warps, st)
-           : D <= 32 ? launch<8, 4, P, CHORD>(a, warps, st)
-           : D <= 64 ? launch<16, 4, P, CHORD>(a, warps, st)
+  if (w8 <= grp::kOnePerWarp && D <= 64)
+    return D <= 32 ? launch<32, 1, P, CHORD>(a, warps, st) : launch<32, 2, P, CHORD>(a, warps, st);
+  if (D <= 16 && (n <= grp::kMid16 || a.R < 16)) return launch<8, 2, P, CHORD>(a, warps, st);
+  if (D <= 32 && D > 16 && (n <= grp::kMid32 || a.R < 16)) return launch<16, 2, P, CHORD>(a, warps, st);
+  if (D <= 16) return launch<4, 4, P, CHORD>(a, warps, st);
+  if (D <= 32) return launch<8, 4, P, CHORD>(a, warps, st);
+  if constexpr (P == 6) {
+    return D <= 64   ? launch<16, 4, P, CHORD>(a, warps, st)
+           : D <= 96 ? launch<32, 3, P, CHORD>(a, warps, st)
                      : launch<32, 4, P, CHORD>(a, warps, st);
-  else
-    return D <= 16   ? launch<4, 4, P, CHORD>(a, warps, st)
-           : D <= 32 ? launch<8, 4, P, CHORD>(a, warps, st)
-           : D <= 48 ? launch<8, 6, P, CHORD, 3>(a, warps, st)
-           : D <= 64 ? launch<16, 4, P, CHORD>(a, warps, st)
-           : D <= 96 ? launch<16, 6, P, CHORD>(a, warps, st)
-                     : launch<16, 8, P, CHORD>(a, warps, st);
+  } else {
+    if (D <= 48) return launch<8, 6, P, CHORD, 3>(a, warps, st);
+    if (D <= 64) return launch<16, 4, P, CHORD>(a, warps, st);
+    return D <= 96 ? launch<16, 6, P, CHORD>(a, warps, st) : launch<16, 8, P, CHORD>(a, warps, st);
+  }
 }
 
 }  // namespace grpf

@@ -614,15 +614,19 @@ static cudaError_t launch_map(const MapParams& a, cudaStream_t st) {
 }
 
 
-constexpr int kReadThreads = 256;
 
 // One block per channel use.  H is staged transposed with a padded stride (Hs[j][i], NR2 + 1) so that the
 // 32 lanes of a warp, which own rows i = lane + 32 m, read consecutive words.  r0 = y - H x_q is formed once;
 // candidate c's residual is r0 - sum_j H[:, j] e_j over the few coordinates where its clipped level differs
 // from the guess (e = x - x_q), and its distance is ||r||^2.
 // MR: rows of H per lane (NR2 <= 32 MR); rows beyond NR2 add exact zeros, so every MR gives the same sums.
-template <int MR>
-__global__ void __launch_bounds__(kReadThreads) k_readout_dd(const ReadParams a) {
+// NT threads: a block's life is mostly waiting (loads, three barriers, serial sums of a few warps), so where the batch
+// fills the GPU smaller blocks, more of them resident, serve it better.  256 threads (small batches, above 64
+// coordinates or 64 candidates) against 32 up to 16 coordinates: 49999 8-user uses 0.58 -> 0.28 ms; 64 up to 32: 16384
+// 16-user uses 0.23 -> 0.15; 128 up to 64: 16384 32-user uses 0.325 -> 0.267; at 128 coordinates 128 threads lose (4096
+// 64-user uses 0.30 -> 0.42).
+template <int MR, int NT>
+__global__ void __launch_bounds__(NT) k_readout_dd(const ReadParams a) {
   extern __shared__ __align__(16) float sm[];
   const int D = a.D, NR2 = a.NR2, P = a.P, R = a.R, b = blockIdx.x;
   const int HS = NR2 + 1;
@@ -632,13 +636,13 @@ __global__ void __launch_bounds__(kReadThreads) k_readout_dd(const ReadParams a)
   float* bd = r0 + NR2;             // 8
   int* br = reinterpret_cast<int*>(bd + 8);  // 8
   int8_t* ek = reinterpret_cast<int8_t*>(br + 8);  // (R + 1) x D: candidate level minus guess; row R = x_q
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, W = kReadThreads / 32;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, W = NT / 32;
   const int lo = 1 - pam_size(a.M), hi = -lo;
   const int u = a.idx ? a.idx[b] : b;
   const float* Hb = a.H + (size_t)u * NR2 * D;
   if ((D & 3) == 0 && (reinterpret_cast<uintptr_t>(Hb) & 15u) == 0) {  // 16-byte loads, four columns of a row
     const float4* H4 = reinterpret_cast<const float4*>(Hb);
-    for (int x = tid; x < NR2 * D / 4; x += kReadThreads) {
+    for (int x = tid; x < NR2 * D / 4; x += NT) {
       const float4 v = H4[x];
       const int i = (4 * x) / D, j = 4 * x - i * D;
       Hs[j * HS + i] = v.x;
@@ -647,13 +651,13 @@ __global__ void __launch_bounds__(kReadThreads) k_readout_dd(const ReadParams a)
       Hs[(j + 3) * HS + i] = v.w;
     }
   } else {
-    for (int x = tid; x < NR2 * D; x += kReadThreads) {
+    for (int x = tid; x < NR2 * D; x += NT) {
       const int i = x / D, j = x - i * D;
       Hs[j * HS + i] = Hb[x];
     }
   }
   int8_t* xq8 = ek + R * D;
-  for (int j = tid; j < D; j += kReadThreads)
+  for (int j = tid; j < D; j += NT)
     xq8[j] = a.mdi ? a.xg[(size_t)u * a.xg_stride + j] : a.xq[(size_t)b * D + j];
   __syncthreads();
   // every candidate's clipped delta from the guess, from one coalesced pass over its spins
@@ -661,7 +665,7 @@ __global__ void __launch_bounds__(kReadThreads) k_readout_dd(const ReadParams a)
   if (!a.ri && (D & 15) == 0 && P <= 6 && (reinterpret_cast<uintptr_t>(sb) & 15u) == 0) {
     // 16 coordinates of one candidate per thread: its P 16-byte spin loads are all in flight at once
     const int ng = D >> 4;
-    for (int x = tid; x < R * ng; x += kReadThreads) {
+    for (int x = tid; x < R * ng; x += NT) {
       const int c = x / ng, j0 = (x - c * ng) << 4;
       int4 sv[6];
 #pragma unroll
@@ -679,7 +683,7 @@ __global__ void __launch_bounds__(kReadThreads) k_readout_dd(const ReadParams a)
       }
     }
   } else {
-    for (int x = tid; x < R * D; x += kReadThreads) {
+    for (int x = tid; x < R * D; x += NT) {
       const int c = x / D, j = x - c * D;
       int xv;
       if (a.ri) {  // RI spins: l = 2 s1 + s2 (16-QAM) or s (QPSK), mimo.spins_to_levels (mimo.py:39-42)
@@ -692,7 +696,7 @@ __global__ void __launch_bounds__(kReadThreads) k_readout_dd(const ReadParams a)
       ek[x] = (int8_t)(xv - xq8[j]);
     }
   }
-  for (int i = tid; i < NR2; i += kReadThreads) {
+  for (int i = tid; i < NR2; i += NT) {
     float r = a.y[(size_t)u * NR2 + i];
     for (int j = 0; j < D; ++j) r = __fmaf_rn(-Hs[j * HS + i], (float)xq8[j], r);
     r0[i] = r;
@@ -798,7 +802,7 @@ __global__ void __launch_bounds__(kReadThreads) k_readout_dd(const ReadParams a)
     float* dn = nj + D;                      // neighbour distances, nbits
     float* rv = dn + nbits;                  // 8 warps x (min1, min2)
     int* ri = reinterpret_cast<int*>(rv + 16);
-    for (int k = tid; k < nbits; k += kReadThreads) s0[k] = s1[k] = __float_as_int(FLT_MAX);
+    for (int k = tid; k < nbits; k += NT) s0[k] = s1[k] = __float_as_int(FLT_MAX);
     __syncthreads();
 #pragma unroll
     for (int m = 0; m < 8; ++m) {
@@ -808,7 +812,7 @@ __global__ void __launch_bounds__(kReadThreads) k_readout_dd(const ReadParams a)
         atomicMin(&s1[k], __float_as_int(mb1[m]));
       }
     }
-    for (int i = tid; i < NR2; i += kReadThreads) {
+    for (int i = tid; i < NR2; i += NT) {
       float r = r0[i];
       if (gi < R)
         for (int j = 0; j < D; ++j)
@@ -816,7 +820,7 @@ __global__ void __launch_bounds__(kReadThreads) k_readout_dd(const ReadParams a)
       rh[i] = r;
     }
     __syncthreads();
-    for (int j = tid; j < D; j += kReadThreads) {
+    for (int j = tid; j < D; j += NT) {
       float c = 0.0f, n = 0.0f;
       for (int i = 0; i < NR2; ++i) {
         const float hv = Hs[j * HS + i];
@@ -829,7 +833,7 @@ __global__ void __launch_bounds__(kReadThreads) k_readout_dd(const ReadParams a)
     __syncthreads();
     float n1 = FLT_MAX, n2 = FLT_MAX;
     int i1 = INT_MAX;
-    for (int k = tid; k < nbits; k += kReadThreads) {
+    for (int k = tid; k < nbits; k += NT) {
       const int j = k / nbl;
       const int lv = xq8[j] + (gi < R ? ek[gi * D + j] : 0);
       // Gray neighbour: the MSB flips the sign; the LSB swaps +-1 and +-3 (16-QAM)
@@ -879,7 +883,7 @@ __global__ void __launch_bounds__(kReadThreads) k_readout_dd(const ReadParams a)
       }
     }
     const float inv_n0 = 1.0f / a.N0[u];
-    for (int k = tid; k < nbits; k += kReadThreads) {
+    for (int k = tid; k < nbits; k += NT) {
       const int j = k / nbl;
       const int lv = xq8[j] + (gi < R ? ek[gi * D + j] : 0);
       const bool bh = (k - j * nbl) == 0 ? lv > 0 : (lv == 1 || lv == -1);
@@ -900,13 +904,13 @@ __global__ void __launch_bounds__(kReadThreads) k_readout_dd(const ReadParams a)
     const float cur = a.bd[(size_t)u * a.bl_stride];
     __syncthreads();
     if (gb < cur) {
-      for (int j = tid; j < D; j += kReadThreads) a.bl[(size_t)u * a.bl_stride * D + j] = (int8_t)(xq8[j] + ek[gi * D + j]);
+      for (int j = tid; j < D; j += NT) a.bl[(size_t)u * a.bl_stride * D + j] = (int8_t)(xq8[j] + ek[gi * D + j]);
       if (tid == 0) a.bd[(size_t)u * a.bl_stride] = gb;
     }
     return;
   }
   const int nb = pam_bits(a.M);
-  for (int j = tid; j < D; j += kReadThreads) {
+  for (int j = tid; j < D; j += NT) {
     const int v = xq8[j] + (gi < R ? ek[gi * D + j] : 0);
     a.levels[(size_t)b * D + j] = (int8_t)v;
     if (nb == 1) {
@@ -947,20 +951,30 @@ static size_t readout_smem(int D, int NR2, int R, bool soft = false) {
   return s;
 }
 
+template <int MR, int NT>
+static cudaError_t launch_readout(const ReadParams& a, size_t smem, cudaStream_t st) {
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(k_readout_dd<MR, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  return launch_ex(k_readout_dd<MR, NT>, dim3(a.B), dim3(NT), smem, st, a.B <= kPdlMaxB, a);
+}
+
+constexpr int kReadSmallB = 148 * 8;  // uses from which small blocks fill the GPU
+
 cudaError_t readout_dispatch(const ReadParams& a, cudaStream_t st) {
   const size_t smem = readout_smem(a.D, a.NR2, a.R, a.llr != nullptr);
-  if (smem > 48 * 1024) {
-    for (auto k : {k_readout_dd<1>, k_readout_dd<2>, k_readout_dd<4>, k_readout_dd<8>}) {
-      cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return e;
-    }
+  if (a.B >= kReadSmallB && a.R <= 64 && a.D <= 64 && a.NR2 <= 128) {
+    if (a.D <= 16 && a.NR2 <= 64)
+      return a.NR2 <= 32 ? launch_readout<1, 32>(a, smem, st) : launch_readout<2, 32>(a, smem, st);
+    if (a.D <= 32 && a.NR2 <= 64)
+      return a.NR2 <= 32 ? launch_readout<1, 64>(a, smem, st) : launch_readout<2, 64>(a, smem, st);
+    return a.NR2 <= 64 ? launch_readout<2, 128>(a, smem, st) : launch_readout<4, 128>(a, smem, st);
   }
-  const bool pdl = a.B <= kPdlMaxB;
-  const dim3 g(a.B), t(kReadThreads);
-  if (a.NR2 <= 32) return launch_ex(k_readout_dd<1>, g, t, smem, st, pdl, a);
-  if (a.NR2 <= 64) return launch_ex(k_readout_dd<2>, g, t, smem, st, pdl, a);
-  if (a.NR2 <= 128) return launch_ex(k_readout_dd<4>, g, t, smem, st, pdl, a);
-  return launch_ex(k_readout_dd<8>, g, t, smem, st, pdl, a);
+  if (a.NR2 <= 32) return launch_readout<1, 256>(a, smem, st);
+  if (a.NR2 <= 64) return launch_readout<2, 256>(a, smem, st);
+  if (a.NR2 <= 128) return launch_readout<4, 256>(a, smem, st);
+  return launch_readout<8, 256>(a, smem, st);
 }
 
 // Workspace of the fused detector call: G, h, x_q, scale, spins, de, (flips, tests), 256-byte aligned.

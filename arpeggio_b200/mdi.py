@@ -66,6 +66,10 @@ def detect(H, y, N0, M, seed, pick, Rmax=None, stages=None, policy='arpeggio', p
     dist = torch.empty(B, G, dtype=torch.float32, device=dev)
     ann = np.zeros(B)
     cnt = counters if counters is not None else {}
+    # the counters stay on the device until the walk is over: per K the sum over the anneals of (flips, tests) and n1,
+    # and the anneals counted here (reading them group by group drained the queue each time: 45 against 39 ms for
+    # 4096 16-user 16-QAM uses)
+    dev_cnt, host_cnt = {}, {}
     seed_base = (seed * 0x9E3779B97F4A7C15) & M64
     calls = 0
     qscale = 1 if precision == 'int' else 0
@@ -117,13 +121,11 @@ def detect(H, y, N0, M, seed, pick, Rmax=None, stages=None, policy='arpeggio', p
                     _lib.check(L.arp_mdi_update(_lib.ptr(H), _lib.ptr(y), _lib.ptr(idx), n, NR2, D, P, na, M,
                                                 _lib.ptr(cur), G, gi, _lib.ptr(spins), _lib.ptr(nxt), _lib.ptr(bd),
                                                 sp), 'mdi_update')
-                    v = cnt.setdefault(str(K), [0, 0, 0] if n1 is None else [0, 0, 0, 0])
-                    s_ = stt.sum((0, 1)).tolist()
-                    v[0] += int(s_[0])
-                    v[1] += int(s_[1])
-                    v[2] += int(na * n)
+                    s_ = stt.sum((0, 1))
                     if n1 is not None:
-                        v[3] += int(n1.sum())
+                        s_ = torch.cat([s_, n1.sum().reshape(1)])
+                    dev_cnt[K] = dev_cnt[K] + s_ if K in dev_cnt else s_
+                    host_cnt[K] = host_cnt.get(K, 0) + na * n
                     ann[idx_np] += na
         cur = nxt
     _lib.check(L.arp_mdi_radius(_lib.ptr(H), _lib.ptr(y), _lib.ptr(cur), B, NR2, D, G, M, Rmax, _lib.ptr(Rd),
@@ -132,6 +134,12 @@ def detect(H, y, N0, M, seed, pick, Rmax=None, stages=None, policy='arpeggio', p
     bits = torch.empty(B, D * PAM[M]['bits'], dtype=torch.int8, device=dev)
     _lib.check(L.arp_mdi_select(_lib.ptr(cur), _lib.ptr(dist), B, D, G, M, _lib.ptr(levels), _lib.ptr(bits), sp),
                'mdi_select')
+    for K, s_ in dev_cnt.items():
+        s_ = s_.tolist()
+        v = cnt.setdefault(str(K), [0] * (len(s_) + 1))
+        for i, x in zip((0, 1, 3), s_):
+            v[i] += int(x)
+        v[2] += int(host_cnt[K])
     torch.cuda.synchronize()
     check_status(status)
     return levels, ann, cnt, bits

@@ -44,6 +44,8 @@ SIGNATURES = {
     'arp_anneal_first_accept_mixed': [_P, _I, _I, _U, _U, _I, _P, _P, _P],
     'arp_map_dd_soft': [_P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _P, _P, _P, _P, _P],
     'arp_gemm_bf16': [_P, _I, _I, _P, _I, _I, _I, _I, _I, _I, _P, _P, _I, _P, _I, _P, _P],
+    'arp_gemm_bf16_ws': [_P, _I, _I, _P, _I, _I, _I, _I, _I, _I, _P, _P, _I, _P, _I, _P, _P, ctypes.c_size_t, _P],
+    'arp_colsum_bf16_ws': [_P, _I, _I, _I, _P, _P, ctypes.c_size_t, _P],
     'arp_warm_features': [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _P, _P],
     'arp_warm_loss': [_P, _I, _P, _I, _I, _P, _I, _P, _P, _P],
     'arp_colsum_bf16': [_P, _I, _I, _I, _P, _P],

@@ -23,6 +23,24 @@ struct GemmParams {
   int ldc;
   int kt_per;  // k tiles (of 64) per split
   int32_t* status;
+  float* ws;  // the caller's workspace for split partials (may be null)
+  size_t ws_bytes;
+};
+
+// Room for the partials of one call: the caller's workspace where it is large enough, else a stream-ordered
+// allocation, which costs the host 15 to 30 us a pair and, after each synchronisation, a new mapping of the memory.
+struct Partials {
+  float* p = nullptr;
+  bool own = false;
+  cudaError_t get(float* ws, size_t ws_bytes, size_t need, cudaStream_t st) {
+    if (ws && ws_bytes >= need) {
+      p = ws;
+      return cudaSuccess;
+    }
+    own = true;
+    return cudaMallocAsync(reinterpret_cast<void**>(&p), need, st);
+  }
+  cudaError_t put(cudaStream_t st) { return own ? cudaFreeAsync(p, st) : cudaSuccess; }
 };
 
 enum { EPI_F32 = 0, EPI_F32_ACC = 1, EPI_BIAS_RELU_BF16 = 2, EPI_BIAS_F32 = 3, EPI_MASK_BF16 = 4 };

@@ -24,11 +24,14 @@ NF, NH, NO = 16, 256, 16
 EPI_F32, EPI_ACC, EPI_RELU_BF16, EPI_BIAS_F32, EPI_MASK_BF16 = range(5)
 
 
-def gemm(A, a_mn, lda, B, b_mn, ldb, M, N, K, epi, C, ldc, bias=None, aux=None, ld_aux=0, status=None, stream=None):
-    """C = A B^T on the tensor cores (arp_gemm_bf16); majors and epilogues as declared in the C header."""
-    _lib.check(_lib.lib().arp_gemm_bf16(_lib.ptr(A), int(a_mn), lda, _lib.ptr(B), int(b_mn), ldb, M, N, K, epi,
-                                        _lib.ptr(bias), _lib.ptr(aux), ld_aux, _lib.ptr(C), ldc, _lib.ptr(status),
-                                        _lib.stream_ptr(stream)), 'gemm_bf16')
+def gemm(A, a_mn, lda, B, b_mn, ldb, M, N, K, epi, C, ldc, bias=None, aux=None, ld_aux=0, status=None, stream=None,
+         ws=None):
+    """C = A B^T on the tensor cores (arp_gemm_bf16); majors and epilogues as declared in the C header.  ws: a float32
+    workspace for the partials of split sums, free for the next call on the same stream."""
+    _lib.check(_lib.lib().arp_gemm_bf16_ws(_lib.ptr(A), int(a_mn), lda, _lib.ptr(B), int(b_mn), ldb, M, N, K, epi,
+                                           _lib.ptr(bias), _lib.ptr(aux), ld_aux, _lib.ptr(C), ldc, _lib.ptr(status),
+                                           _lib.ptr(ws), 0 if ws is None else 4 * ws.numel(),
+                                           _lib.stream_ptr(stream)), 'gemm_bf16')
 
 
 class WarmMLP:
@@ -85,6 +88,9 @@ class WarmMLP:
             self.dZ3 = torch.empty(rows, NO, dtype=b16, device=dev)
             self.dZ2 = torch.empty(rows, NH, dtype=b16, device=dev)
             self.dZ1 = torch.empty(rows, NH, dtype=b16, device=dev)
+            # partials of the gradients' split sums (the widest: 74 splits of a 256 x 256 gradient); allocated per
+            # call they cost the step 0.5 ms when it runs alone, the memory being mapped again after each sync
+            self.part = torch.empty(80 * NH * NH, dtype=torch.float32, device=dev)
             self._train = True
         self._rows = rows
 
@@ -130,18 +136,24 @@ class WarmMLP:
         _lib.check(L.arp_warm_loss(_lib.ptr(self.Z), NO, _lib.ptr(labels), rows, self.C, _lib.ptr(self.dZ3), NO,
                                    _lib.ptr(self.loss), _lib.ptr(self.correct), sp), 'warm_loss')
         g = self.grad
+
+        def colsum(X, cols, name):
+            _lib.check(L.arp_colsum_bf16_ws(_lib.ptr(X), rows, cols, cols, _lib.ptr(self.view(g, name)),
+                                            _lib.ptr(self.part), 4 * self.part.numel(), sp), 'colsum')
+
         gemm(self.H2, 1, NH, self.dZ3, 1, NO, NH, NO, rows, EPI_ACC, self.view(g, 'W3t'), NO, status=st,
-             stream=stream)
-        _lib.check(L.arp_colsum_bf16(_lib.ptr(self.dZ3), rows, NO, NO, _lib.ptr(self.view(g, 'b3')), sp), 'colsum')
+             stream=stream, ws=self.part)
+        colsum(self.dZ3, NO, 'b3')
         gemm(self.dZ3, 0, NO, self.view(self.wb, 'W3t'), 0, NO, rows, NH, NO, EPI_MASK_BF16, self.dZ2, NH,
              aux=self.H2, ld_aux=NH, status=st, stream=stream)
         gemm(self.dZ2, 1, NH, self.H1, 1, NH, NH, NH, rows, EPI_ACC, self.view(g, 'W2'), NH, status=st,
-             stream=stream)
-        _lib.check(L.arp_colsum_bf16(_lib.ptr(self.dZ2), rows, NH, NH, _lib.ptr(self.view(g, 'b2')), sp), 'colsum')
+             stream=stream, ws=self.part)
+        colsum(self.dZ2, NH, 'b2')
         gemm(self.dZ2, 0, NH, self.view(self.wb, 'W2'), 1, NH, rows, NH, NH, EPI_MASK_BF16, self.dZ1, NH,
              aux=self.H1, ld_aux=NH, status=st, stream=stream)
-        gemm(self.dZ1, 1, NH, X, 1, NF, NH, NF, rows, EPI_ACC, self.view(g, 'W1'), NF, status=st, stream=stream)
-        _lib.check(L.arp_colsum_bf16(_lib.ptr(self.dZ1), rows, NH, NH, _lib.ptr(self.view(g, 'b1')), sp), 'colsum')
+        gemm(self.dZ1, 1, NH, X, 1, NF, NH, NF, rows, EPI_ACC, self.view(g, 'W1'), NF, status=st, stream=stream,
+             ws=self.part)
+        colsum(self.dZ1, NH, 'b1')
 
     def adam(self, scale, lr=1e-3, beta1=0.9, beta2=0.999, eps=1e-8, stream=None):
         self.steps += 1

@@ -270,14 +270,23 @@ int arp_map_dd_soft(const float* H, const float* y, const float* sigma2, int B, 
  * A is (M, K) row-major with row stride lda (a_mn_major = 0) or (K, M) row-major (a_mn_major = 1); B is (N, K)
  * (b_mn_major = 0) or (K, N) (b_mn_major = 1).  N and K multiples of 16, leading dimensions multiples of 8
  * elements, pointers 16-byte aligned.  epilogue: 0 C = acc (float), 1 C += acc (float; K is split over CTAs
- * whose partial products go to a stream-ordered workspace and are added in split order, so the result is the
+ * whose partial products go to a stream-ordered workspace and are added in a fixed order, so the result is the
  * same on every run), 2 C = bf16(max(acc + bias, 0)), 3 C = acc + bias (float), 4 C = bf16(acc if aux > 0 else
- * 0) with aux (M, N) bf16 of row stride ld_aux (the ReLU backward).  Products with M >= 128, N >= 64 and K >= 64
- * run on a persistent kernel fed by TMA tensor loads with warp-specialised producer, MMA and epilogue roles; the
- * rest on a cp.async-fed kernel.  Either way each shape gives the same result on every run. */
+ * 0) with aux (M, N) bf16 of row stride ld_aux (the ReLU backward).  Products with M >= 128 (epilogue 1: also
+ * N >= 64 and K >= 64) run on a persistent kernel fed by TMA tensor loads with warp-specialised producer, MMA and
+ * epilogue roles; the rest on a cp.async-fed kernel.  Either way each shape gives the same result on every run. */
 int arp_gemm_bf16(const void* A, int a_mn_major, int lda, const void* B, int b_mn_major, int ldb, int M, int N, int K,
                   int epilogue, const float* bias, const void* aux, int ld_aux, void* C, int ldc, int32_t* status,
                   void* stream);
+
+/* arp_gemm_bf16 and arp_colsum_bf16 with the caller's workspace (ws_bytes at ws, 16-byte aligned or NULL) for the
+ * partials of a split sum; where it is too small or NULL the partials take a stream-ordered allocation.  The
+ * workspace may be reused by the next call on the same stream. */
+int arp_gemm_bf16_ws(const void* A, int a_mn_major, int lda, const void* B, int b_mn_major, int ldb, int M, int N,
+                     int K, int epilogue, const float* bias, const void* aux, int ld_aux, void* C, int ldc,
+                     int32_t* status, void* ws, size_t ws_bytes, void* stream);
+int arp_colsum_bf16_ws(const void* X, int rows, int cols, int ld, float* out, void* ws, size_t ws_bytes,
+                       void* stream);
 
 /* Per-coordinate features X (B*D, 16) bf16 of mapped dDI problems G (B, D, D), h (B, D) (int32 when quantized,
  * else float), guesses xq (B, D), MMSE soft estimates zs (B, D) (may be NULL), snr_db (B) (may be NULL).  With

@@ -46,6 +46,7 @@ SIGNATURES = {
     'arp_gemm_bf16': [_P, _I, _I, _P, _I, _I, _I, _I, _I, _I, _P, _P, _I, _P, _I, _P, _P],
     'arp_gemm_bf16_ws': [_P, _I, _I, _P, _I, _I, _I, _I, _I, _I, _P, _P, _I, _P, _I, _P, _P, ctypes.c_size_t, _P],
     'arp_colsum_bf16_ws': [_P, _I, _I, _I, _P, _P, ctypes.c_size_t, _P],
+    'arp_mlp_train_step': [_P, _P, _I, _I] + [_P] * 13 + [ctypes.c_size_t, _P, _P, _F, _F, _F, _F, _I, _P, _P],
     'arp_warm_features': [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _P, _P],
     'arp_warm_loss': [_P, _I, _P, _I, _I, _P, _I, _P, _P, _P],
     'arp_colsum_bf16': [_P, _I, _I, _I, _P, _P],

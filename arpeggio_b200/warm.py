@@ -165,9 +165,15 @@ class WarmMLP:
     def train_step(self, X, labels, rows, lr=1e-3, stream=None):
         """Forward, backward and one Adam step on the mean loss over `rows` rows (a multiple of 16)."""
         self.reserve(rows, train=True)
-        self.forward(X, rows, stream)
-        self.backward(X, labels, rows, stream)
-        self.adam(1.0 / rows, lr, stream=stream)
+        if rows % 16:
+            raise ValueError('rows must be a multiple of 16')
+        p = _lib.ptr
+        _lib.check(_lib.lib().arp_mlp_train_step(
+            p(X), p(labels), rows, self.C, p(self.w), p(self.wb), p(self.w2p), p(self.grad), p(self.m), p(self.v),
+            p(self.H1), p(self.H2), p(self.Z), p(self.dZ3), p(self.dZ2), p(self.dZ1), p(self.part),
+            4 * self.part.numel(), p(self.loss), p(self.correct), float(lr), 0.9, 0.999, 1e-8, self.steps + 1,
+            p(self.status), _lib.stream_ptr(stream)), 'mlp_train_step')
+        self.steps += 1
 
     def check(self):
         _lib.check(int(self.status.item()), 'warm MLP')

@@ -308,6 +308,15 @@ int arp_colsum_bf16(const void* X, int rows, int cols, int ld, float* out, void*
 int arp_adam(float* w, void* w_bf16, const float* grad, float* m, float* v, int n, float lr, float beta1, float beta2,
              float eps, int step, float grad_scale, void* stream);
 
+/* One optimisation step of the warm start's network (16 -> 256 -> 256 -> 16, ReLU) on the mean loss over `rows` rows
+ * (a multiple of 16): forward, loss, gradients, Adam and the packed copy of W2, as the entries above and
+ * arp_mlp_pack_w2 do them one by one.  w, grad, m, v (float) and w_bf16 hold W1 (256, 16), b1, W2 (256, 256), b2,
+ * W3t (256, 16), b3 in this order; H1, H2, dZ2, dZ1 (rows, 256) and dZ3 (rows, 16) bf16, Z (rows, 16) float. */
+int arp_mlp_train_step(const void* X, const int8_t* labels, int rows, int classes, float* w, void* w_bf16,
+                       void* w2_packed, float* grad, float* m, float* v, void* H1, void* H2, float* Z, void* dZ3,
+                       void* dZ2, void* dZ1, void* ws, size_t ws_bytes, float* loss_sum, int32_t* correct, float lr,
+                       float beta1, float beta2, float eps, int step, int32_t* status, void* stream);
+
 /* W2 (256, 256) bf16 row-major -> W2p, the same 256 x 256 values in the order arp_mlp_forward keeps them in
  * shared memory (8 chunks of 256 rows x 32 k; within a chunk k-group of 8, then row, then element).  Once per
  * weight update. */

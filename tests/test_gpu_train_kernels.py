@@ -83,3 +83,23 @@ def test_column_sums(rows, cols, ld, off):
     tol = (rows + 1) * 2.0 ** -24 * (1 + X[:, :cols].double().abs().sum(0))
     assert bool(((outs[0].double() - ref).abs() <= tol).all())
     assert torch.equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize('rows,P', [(16, 2), (1008, 4), (20000, 6)])
+def test_one_call_step_is_the_steps_one_by_one(rows, P):
+    from arpeggio_b200 import warm
+    g = torch.Generator().manual_seed(rows)
+    X = _bf((rows, 16), g)
+    labels = torch.randint(-1, P + 1, (rows,), generator=g).to(torch.int8).cuda()
+    a, b = warm.WarmMLP(P=P, seed=3), warm.WarmMLP(P=P, seed=3)
+    for _ in range(3):
+        a.train_step(X, labels, rows, lr=2e-3)
+        b.reserve(rows, train=True)
+        b.forward(X, rows)
+        b.backward(X, labels, rows)
+        b.adam(1.0 / rows, 2e-3)
+    torch.cuda.synchronize()
+    for k in ('w', 'wb', 'm', 'v', 'grad', 'w2p', 'correct'):
+        assert torch.equal(getattr(a, k), getattr(b, k)), k
+    torch.testing.assert_close(a.loss, b.loss, rtol=1e-5, atol=0)  # a sum of float atomics
+    assert a.steps == b.steps == 3

@@ -399,33 +399,62 @@ __global__ void __launch_bounds__(128) k_warm_features(const GT* __restrict__ G,
 }
 
 // ------------------------------------------------------------------------------------------------ loss
+// One thread per row (at most eight classes, in registers).  Bound by its sums' atomics and its stores: one pair of
+// atomics per block instead of per warp, and the 32-byte gradient row (wide = 1: ldd = 16, aligned) in two stores
+// instead of sixteen.  One training step of 65,536 rows 234 -> 224 us.
 __global__ void __launch_bounds__(256) k_warm_loss(const float* __restrict__ logits, int ldl,
                                                    const int8_t* __restrict__ labels, int rows, int C,
-                                                   bf16* __restrict__ dl, int ldd, float* loss_sum, int* correct) {
+                                                   bf16* __restrict__ dl, int ldd, int wide, float* loss_sum,
+                                                   int* correct) {
+  __shared__ float s_l[8];
+  __shared__ int s_ok[8];
   const int row = blockIdx.x * blockDim.x + threadIdx.x;
   float l = 0.0f;
   int ok = 0;
   if (row < rows) {
-    const float* z = logits + (size_t)row * ldl;
+    float z[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) z[c] = c < C ? logits[(size_t)row * ldl + c] : 0.0f;
+    const int lab = labels[row];
+    const float zl = lab >= 0 ? logits[(size_t)row * ldl + lab] : 0.0f;
     float zm = -INFINITY;
     int am = 0;
-    for (int c = 0; c < C; ++c)
-      if (z[c] > zm) {
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      if (c < C && z[c] > zm) {
         zm = z[c];
         am = c;
       }
+    }
     float se = 0.0f;
-    for (int c = 0; c < C; ++c) se += __expf(z[c] - zm);
-    const int lab = labels[row];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      z[c] = __expf(z[c] - zm);
+      if (c < C) se += z[c];
+    }
     if (lab >= 0) {
-      l = __logf(se) + zm - z[lab];
+      l = __logf(se) + zm - zl;
       ok = am == lab;
     }
-    bf16* g = dl + (size_t)row * ldd;
-    for (int c = 0; c < ldd; ++c) {
-      float v = 0.0f;
-      if (c < C && lab >= 0) v = __expf(z[c] - zm) / se - (c == lab ? 1.0f : 0.0f);
-      g[c] = __float2bfloat16_rn(v);
+    uint32_t g[4];
+#pragma unroll
+    for (int c = 0; c < 8; c += 2) {
+      float v[2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) v[i] = c + i < C && lab >= 0 ? z[c + i] / se - (c + i == lab ? 1.0f : 0.0f) : 0.0f;
+      const __nv_bfloat162 h2 = __floats2bfloat162_rn(v[0], v[1]);
+      g[c / 2] = *reinterpret_cast<const uint32_t*>(&h2);
+    }
+    if (wide) {
+      uint4* o = reinterpret_cast<uint4*>(dl + (size_t)row * 16);
+      o[0] = make_uint4(g[0], g[1], g[2], g[3]);
+      o[1] = make_uint4(0u, 0u, 0u, 0u);
+    } else {
+      unsigned short* o = reinterpret_cast<unsigned short*>(dl + (size_t)row * ldd);
+#pragma unroll
+      for (int c = 0; c < 8; ++c)
+        if (c < ldd) o[c] = (unsigned short)(c % 2 ? g[c / 2] >> 16 : g[c / 2] & 0xFFFFu);
+      for (int c = 8; c < ldd; ++c) o[c] = 0;
     }
   }
 #pragma unroll
@@ -434,6 +463,16 @@ __global__ void __launch_bounds__(256) k_warm_loss(const float* __restrict__ log
     ok += __shfl_xor_sync(0xffffffffu, ok, o);
   }
   if ((threadIdx.x & 31) == 0) {
+    s_l[threadIdx.x >> 5] = l;
+    s_ok[threadIdx.x >> 5] = ok;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int i = 1; i < 8; ++i) {
+      l += s_l[i];
+      ok += s_ok[i];
+    }
     if (loss_sum) atomicAdd(loss_sum, l);
     if (correct) atomicAdd(correct, ok);
   }
@@ -952,8 +991,8 @@ extern "C" int arp_warm_loss(const float* logits, int ldl, const int8_t* labels,
   if (rows < 0 || classes < 2 || classes > ldl || classes > ldd || classes > 8) return ARP_ERR_SHAPE;
   if (rows == 0) return ARP_OK;
   if (!logits || !labels || !dlogits) return ARP_ERR_ARG;
-  k_warm_loss<<<(rows + 255) / 256, 256, 0, (cudaStream_t)stream>>>(logits, ldl, labels, rows, classes, (bf16*)dlogits,
-                                                                    ldd, loss_sum, correct);
+  k_warm_loss<<<(rows + 255) / 256, 256, 0, (cudaStream_t)stream>>>(
+      logits, ldl, labels, rows, classes, (bf16*)dlogits, ldd, ldd == 16 && al16(dlogits), loss_sum, correct);
   return cudaGetLastError() == cudaSuccess ? ARP_OK : ARP_ERR_LAUNCH;
 }
 

@@ -103,3 +103,30 @@ def test_one_call_step_is_the_steps_one_by_one(rows, P):
         assert torch.equal(getattr(a, k), getattr(b, k)), k
     torch.testing.assert_close(a.loss, b.loss, rtol=1e-5, atol=0)  # a sum of float atomics
     assert a.steps == b.steps == 3
+
+
+@pytest.mark.parametrize('rows,classes,ldl,ldd,off', [(1, 2, 5, 3, 0), (255, 3, 16, 16, 0), (1000, 8, 8, 9, 0),
+                                                      (513, 7, 16, 16, 1), (257, 5, 12, 24, 0)])
+def test_loss(rows, classes, ldl, ldd, off):
+    """Softmax cross-entropy and its gradient against float64: __expf is off by at most 2 + 1.2 |x| units in the last
+    place, |x| <= 30 here, the quotient and the difference by one each, the bf16 store by 2^-8."""
+    from arpeggio_b200 import _lib
+    g = torch.Generator().manual_seed(rows)
+    z = (torch.rand(rows, ldl, generator=g) * 30 - 15).cuda()
+    lab = torch.randint(-1, classes, (rows,), generator=g).to(torch.int8).cuda()
+    flat = torch.full((rows * ldd + 8,), 7.0, dtype=torch.bfloat16, device='cuda')
+    d = flat[off:off + rows * ldd].view(rows, ldd)
+    loss, hits = torch.zeros(1, device='cuda'), torch.zeros(1, dtype=torch.int32, device='cuda')
+    _lib.check(_lib.lib().arp_warm_loss(_lib.ptr(z), ldl, _lib.ptr(lab), rows, classes, _lib.ptr(d), ldd,
+                                        _lib.ptr(loss), _lib.ptr(hits), _lib.stream_ptr()), 'loss')
+    torch.cuda.synchronize()
+    zc, use = z[:, :classes].double(), (lab >= 0)
+    pr = torch.softmax(zc, 1)
+    hot = torch.nn.functional.one_hot(lab.clamp(min=0).long(), classes).double()
+    ref = torch.where(use[:, None], pr - hot, 0)
+    assert bool(((d[:, :classes].double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 90 * 2.0 ** -23 * pr).all())
+    assert bool((d[:, classes:] == 0).all())
+    per = torch.where(use, torch.logsumexp(zc, 1) - (zc * hot).sum(1), 0)
+    assert abs(loss.item() - per.sum().item()) <= 1e-5 * (per.abs().sum().item() + rows)
+    assert int(hits.item()) == int((use & (zc.argmax(1) == lab)).sum())
+    assert bool((flat[off + rows * ldd:] == 7).all()) and bool((flat[:off] == 7).all())

@@ -726,8 +726,14 @@ static cudaError_t dispatch(const DDParams& a, int warps, cudaStream_t st) {
   const long long n = (long long)a.B * a.R, w8 = (long long)a.B * ((a.R + 7) / 8 * 8);
   // (above 64 coordinates an unbounded block fills the SM's registers, half the warps; there, or with few anneals a use,
   // which would leave two anneals per warp too few warps beside 64 KB of G, one per warp at 128 registers)
+  // Two anneals per warp fill the GPU with 2 kLatWarps of them, one per warp with half as many: just above a whole number
+  // of the first's waves the finer steps of the second leave less of the last wave empty (5000 to 7100 anneals of 126
+  // coordinates: Chord 248 -> 230 us, first accept 264 -> 253; of 90 coordinates 177 -> 168), at 64 anneals a use also
+  // above the second wave (9600 to 14000: 431 -> 390, 275 -> 260; at 32 a use 386 against 396, so not there).
+  const bool ragged = (w8 > 2 * kLatWarps && w8 <= 3 * kLatWarps) ||
+                      (a.R >= 64 && w8 > 4 * kLatWarps && w8 <= 6 * kLatWarps);
   if constexpr (RULE != kEngine && P < 6)
-    if (D > 64 && w8 > kLatWarps / 2 && (w8 <= kLatWarps || a.R < 16))
+    if (D > 64 && w8 > kLatWarps / 2 && (w8 <= kLatWarps || ragged || a.R < 16))
       return D <= 96 ? launch<32, 3, P, RULE>(a, warps, st) : launch<32, 4, P, RULE>(a, warps, st);
   if (RULE != kEngine && w8 <= (D > 64 ? kLatWarps / 2 : kLatWarps))
     return D <= 32   ? launch<32, 1, P, RULE, 1>(a, warps, st)
@@ -746,6 +752,9 @@ static cudaError_t dispatch(const DDParams& a, int warps, cudaStream_t st) {
            : D <= 96 ? launch<32, 3, P, RULE>(a, warps, st)
                      : launch<32, 4, P, RULE>(a, warps, st);
   } else {
+    // (warm-started anneals: most problems run a few anneals each, which four to a warp would leave on one warp of the
+    // block; 32768 32-user uses 8.28 -> 7.99 ms, 2741 uses 0.84 -> 0.78)
+    if (D <= 64 && D > 48 && RULE == kWarm && a.R < 64) return launch<16, 4, P, RULE>(a, warps, st);
     if (D <= 64 && (n <= kMid64 || a.R < 16)) return launch<16, 4, P, RULE>(a, warps, st);
     return D <= 48   ? launch<8, 6, P, RULE>(a, warps, st)
            : D <= 64 ? launch<8, 8, P, RULE>(a, warps, st)

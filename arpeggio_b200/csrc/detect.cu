@@ -1,6 +1,6 @@
 // Detector stages around the anneal: Gram/field formation with the MMSE guess (map) and the readout.
 //
-// map (one block per channel use; mimo.py:98-109 mmse, :176-182 _mu, :86-88 quantize_levels,
+// map (one to four channel uses per block; mimo.py:98-109 mmse, :176-182 _mu, :86-88 quantize_levels,
 // :506-523 ising_delta_at, chordfx.py:60-76 to_fixed, chord_ref.py:47-59 compress):
 //   Q = H^T H on the tensor cores, exactly: per use H is scaled by a power of two so that its largest entry
 //   is just below 2^30, rounded to integers x and split into four signed 8-bit digits (x = sum_a 2^(8a) d_a);

@@ -722,7 +722,7 @@ def run_ours(args):
         'stages_ms': {'map': stage[0], 'anneal': stage[1], 'readout': stage[2]},
         'roofline': {'bound': 'int_issue', 'achieved': ops / t_anneal / 1e9, 'peak': peak_ops / 1e9,
                      'unit': 'Gop/s', 'frac': ops / t_anneal / peak_ops, 'traffic': traffic,
-                     'kernel': 'k_anneal_int<2, 2, first accept, cached Philox>',
+                     'kernel': 'k_anneal_grp<8, 8, 2, first accept>',
                      'ops_model': '100 per Philox4x32-10 block + 5 per lane decision + 3 per field update',
                      'peak_source': 'measured in this run: arp_philox_rate (chained Philox blocks, all SMs); '
                                     'MEASURED_PEAKS.json has no integer peak'},

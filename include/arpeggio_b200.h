@@ -3,7 +3,8 @@
  *
  * Plain pointers and sizes; every array argument is DEVICE memory unless stated otherwise.  No entry
  * point of the detection path allocates memory; two training routines take stream-ordered workspaces
- * (cudaMallocAsync, freed on the same stream): arp_gemm_bf16 with split K and arp_colsum_bf16.  Every entry
+ * (cudaMallocAsync, freed on the same stream) unless the caller gives one: arp_gemm_bf16 with split K and
+ * arp_colsum_bf16 (the _ws forms and arp_mlp_train_step take the caller's).  Every entry
  * point is stream-ordered on `stream` (a cudaStream_t, or NULL for the legacy default stream) and returns
  * without synchronising, except arp_serve_run, a host loop that returns when its requests are done.  Return value: ARP_OK or an
  * ARP_ERR_* code for errors found on the host (shapes, arguments, launch).  Errors that only the

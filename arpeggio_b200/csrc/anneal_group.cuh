@@ -724,16 +724,19 @@ template <int P, Rule RULE>
 static cudaError_t dispatch(const DDParams& a, int warps, cudaStream_t st) {
   const int D = a.D;
   const long long n = (long long)a.B * a.R, w8 = (long long)a.B * ((a.R + 7) / 8 * 8);
-  // (above 64 coordinates an unbounded block fills the SM's registers, half the warps; there, or with few anneals a use,
-  // which would leave two anneals per warp too few warps beside 64 KB of G, one per warp at 128 registers)
+  // (above 64 coordinates an unbounded block fills the SM's registers, half the warps; there one per warp at 128 registers)
   // Two anneals per warp fill the GPU with 2 kLatWarps of them, one per warp with half as many: just above a whole number
   // of the first's waves the finer steps of the second leave less of the last wave empty (5000 to 7100 anneals of 126
   // coordinates: Chord 248 -> 230 us, first accept 264 -> 253; of 90 coordinates 177 -> 168), at 64 anneals a use also
   // above the second wave (9600 to 14000: 431 -> 390, 275 -> 260; at 32 a use 386 against 396, so not there).
   const bool ragged = (w8 > 2 * kLatWarps && w8 <= 3 * kLatWarps) ||
                       (a.R >= 64 && w8 > 4 * kLatWarps && w8 <= 6 * kLatWarps);
+  // And so for a count that fills its last block of 16 badly, at any size: 34000 anneals of 90 coordinates, 33 a use, Chord
+  // 1200 -> 1060 us, first accept 1510 -> 1365; below 16 a use there are too few warps beside 64 KB of G.
+  const bool waste = (a.R + 15) / 16 * 128 > a.R * 9;
+  const bool start = RULE == kChord && w8 <= kLatWarps * 5 / 4;  // just above one per warp's first wave: 224 -> 207 us
   if constexpr (RULE != kEngine && P < 6)
-    if (D > 64 && w8 > kLatWarps / 2 && (w8 <= kLatWarps || ragged || a.R < 16))
+    if (D > 64 && w8 > kLatWarps / 2 && (w8 <= kLatWarps || ragged || waste || start))
       return D <= 96 ? launch<32, 3, P, RULE>(a, warps, st) : launch<32, 4, P, RULE>(a, warps, st);
   if (RULE != kEngine && w8 <= (D > 64 ? kLatWarps / 2 : kLatWarps))
     return D <= 32   ? launch<32, 1, P, RULE, 1>(a, warps, st)

@@ -501,18 +501,22 @@ __device__ __forceinline__ void problem(const DDParams& a, const PhiloxKeys& K, 
   const int x1 = threadIdx.x;
   const int32_t h1 = x1 < D ? hg[x1] : 0, t1 = x1 < L ? Tg[x1] : 0, c1 = (CHORD && cg && x1 < L) ? cg[x1] : 0;
   const uint32_t inst = a.inst ? a.inst[b] : a.inst0 + (uint32_t)b;
+  bool order = true;  // every thread's: perm is an order of 0..D-1
   if constexpr (WARM) {
-    // position j' of the scan holds coordinate perm[j']: G and h are gathered into that order
-    for (int x = threadIdx.x; x < 128; x += bt) s_inv[x] = 0;
-    __syncthreads();
+    // position j' of the scan holds coordinate perm[j']: G goes into that order by the inverse, h is gathered
     for (int x = threadIdx.x; x < D; x += bt) {
       const uint8_t pv = a.perm[(size_t)b * D + x];
-      if (pv >= D) s_bad = 1;  // not an order of 0..D-1: reported as ARP_ERR_RANGE, never dereferenced
+      bad |= pv >= D;  // reported as ARP_ERR_RANGE, never dereferenced
       s_perm[x] = pv < D ? pv : 0;
       if (pv < D) s_inv[pv] = (uint8_t)x;
     }
+    __syncthreads();
+    bool off = bad;
+    for (int x = threadIdx.x; x < D; x += bt) off |= s_inv[s_perm[x]] != x;
+    order = !__syncthreads_or(off);
+  } else {
+    __syncthreads();
   }
-  __syncthreads();
   auto put = [&](int j, int i, int32_t g) {  // G[j][i] into its place (WARM: in the scan order)
     if constexpr (WARM) {
       j = s_inv[j];
@@ -521,7 +525,17 @@ __device__ __forceinline__ void problem(const DDParams& a, const PhiloxKeys& K, 
     mg = max(mg, (uint32_t)abs(g));
     Gs[j * DP + row_pos<LN, C>(i / LN, LN - 1 - (i & (LN - 1)))] = g;
   };
-  for (int x0 = threadIdx.x; x0 < nv; x0 += 8 * bt) {
+  if (WARM && !order) {
+    // repeated entries: no inverse (s_inv has places that were never written), so G is gathered, entry by entry
+#pragma unroll 1
+    for (int x = threadIdx.x; x < D * D; x += bt) {
+      const int j = x / D, i = x - j * D;
+      const int32_t g = Gg[(int)s_perm[j] * D + s_perm[i]];
+      mg = max(mg, (uint32_t)abs(g));
+      Gs[j * DP + row_pos<LN, C>(i / LN, LN - 1 - (i & (LN - 1)))] = g;
+    }
+  }
+  for (int x0 = order ? (int)threadIdx.x : nv; x0 < nv; x0 += 8 * bt) {
     if (x0 != (int)threadIdx.x) fetch(x0);
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
@@ -537,7 +551,7 @@ __device__ __forceinline__ void problem(const DDParams& a, const PhiloxKeys& K, 
   if constexpr (LN == 32) {
     const int lane = threadIdx.x & 31, W = bt >> 5;
 #pragma unroll 1
-    for (int j0 = threadIdx.x >> 5; j0 < D; j0 += 4 * W) {
+    for (int j0 = order ? (int)threadIdx.x >> 5 : D; j0 < D; j0 += 4 * W) {
       int32_t g[4][C];
 #pragma unroll
       for (int u = 0; u < 4; ++u)
@@ -550,7 +564,7 @@ __device__ __forceinline__ void problem(const DDParams& a, const PhiloxKeys& K, 
         for (int c = 0; c < C; ++c)
           if (j0 + u * W < D && c * 32 + lane < D) put(j0 + u * W, c * 32 + lane, g[u][c]);
     }
-  } else if (!vec) {
+  } else if (!vec && order) {
     for (int x = threadIdx.x; x < D * D; x += bt) put(x / D, x % D, Gg[x]);
   }
   for (int x = threadIdx.x; x < D * (DP - D); x += bt) {  // padding columns

@@ -113,6 +113,11 @@ __device__ __forceinline__ void run(const DDParams& a, const PhiloxKeys& K, cons
   // 1024 uses); where 64 registers are the limit it loses (32 users: 2.94 -> 3.51 ms per 8192 uses).
   constexpr bool AHEAD = LN == 32 && !WIDE;
   constexpr bool HOIST = LN == 4 || LN * C > 64;
+  // One anneal per warp: where its latency is what counts (up to two coordinates a lane), or the reduction would be of
+  // 64 bits (five steps of two shuffles), a flip's psi goes to every lane by a shuffle beside its factor's and no
+  // reduction stands between one pass and the next.  64 sweeps, chain of map, anneal and readout, with the reduction
+  // against without: one 32-user frame 86.9 -> 81.4 us, one 8-user frame 37.1 -> 33.9, 40 9-user frames 58.9 -> 53.7.
+  constexpr bool SPREAD = LN == 32 && (WIDE || C <= 2);
   static_assert(P * C <= 32, "a lane's spins are one 32-bit word");
   static_assert(!ENG || WIDE, "the engine's numbers have no stored thresholds");
   using ET = typename std::conditional<WIDE, long long, int32_t>::type;
@@ -310,7 +315,10 @@ __device__ __forceinline__ void run(const DDParams& a, const PhiloxKeys& K, cons
             load_row<LN, C>(g0 + c * LN * DP * 4 - (uint32_t)l * (DP * 4), ln, g);
 #pragma unroll
             for (int t = 0; t < C; ++t) w[t] += so4 * g[t];
-            if (lane == l) {
+            if constexpr (SPREAD) {
+              de += __shfl_sync(ARP_FULL, psi, l);
+              if (lane == l) fb |= 1u << (p * C + c);
+            } else if (lane == l) {
               if constexpr (WIDE)
                 e = mad_wide_s32(psi, 1, e);
               else
@@ -318,7 +326,7 @@ __device__ __forceinline__ void run(const DDParams& a, const PhiloxKeys& K, cons
               fb |= 1u << (p * C + c);
             }
             jl = l;
-            if constexpr (LN == 32) any = true;
+            if constexpr (LN == 32 && !SPREAD) any = true;
           };
           if constexpr (!CHORD && HOIST) {
             int32_t x[C], zs = 0;
@@ -374,34 +382,41 @@ __device__ __forceinline__ void run(const DDParams& a, const PhiloxKeys& K, cons
               const int32_t z = (w[c] + x) ^ sm;
               if (z < 0) snap |= 1u << c;
             }
+            uint32_t mb[C], ma = 0;  // one anneal per warp: the slots' ballots at once, a quiet pass takes one branch
+            if constexpr (SPREAD) {
 #pragma unroll
-            for (int c = 0; c < C; ++c) {
-              const int32_t sm = -(int32_t)((dn >> (p * C + c)) & 1u);
-              const int32_t s4 = (sm & -8) ^ 4;
-              const bool sn = (snap >> c) & 1u;
-              int jl = 32;
-              if constexpr (LN == 32) {  // one anneal: its flips are the ballot's bits
-                for (uint32_t m = __ballot_sync(ARP_FULL, sn); m != 0; m &= (1u << jl) - 1u)
-                  commit(c, true, m, s4, (w[c] ^ sm) - sm + dg[c] - 1, jl);  // psi = s w + 2 G_jj
-              } else {
-                for (;;) {
-                  const bool acc = sn && lane < jl;
-                  const uint32_t m = __ballot_sync(ARP_FULL, acc);
-                  if (m == 0) break;
-                  commit(c, acc, m, s4, (w[c] ^ sm) - sm + dg[c] - 1, jl);
+              for (int c = 0; c < C; ++c) ma |= mb[c] = __ballot_sync(ARP_FULL, (snap >> c) & 1u);
+            }
+            if (!SPREAD || ma != 0) {
+#pragma unroll
+              for (int c = 0; c < C; ++c) {
+                const int32_t sm = -(int32_t)((dn >> (p * C + c)) & 1u);
+                const int32_t s4 = (sm & -8) ^ 4;
+                const bool sn = (snap >> c) & 1u;
+                int jl = 32;
+                if constexpr (LN == 32) {  // one anneal: its flips are the ballot's bits
+                  for (uint32_t m = SPREAD ? mb[c] : __ballot_sync(ARP_FULL, sn); m != 0; m &= (1u << jl) - 1u)
+                    commit(c, true, m, s4, (w[c] ^ sm) - sm + dg[c] - 1, jl);  // psi = s w + 2 G_jj
+                } else {
+                  for (;;) {
+                    const bool acc = sn && lane < jl;
+                    const uint32_t m = __ballot_sync(ARP_FULL, acc);
+                    if (m == 0) break;
+                    commit(c, acc, m, s4, (w[c] ^ sm) - sm + dg[c] - 1, jl);
+                  }
                 }
               }
             }
             if (a.out_n1) n1 += (__ballot_sync(ARP_FULL, (fb >> (p * C)) != 0) & gmask) != 0;
           }
-          if (any) {
-            if constexpr (LN == 32 && !WIDE) {
-              e = __reduce_add_sync(ARP_FULL, e);
-            } else {
+          if (SPREAD || any) {
+            if constexpr (LN == 32 && !SPREAD) {
+              de += __reduce_add_sync(ARP_FULL, e);
+            } else if constexpr (!SPREAD) {
 #pragma unroll
               for (int o = LN / 2; o; o >>= 1) e += __shfl_xor_sync(ARP_FULL, e, o);
+              de += e;
             }
-            de += e;
             if (de < best) {  // best state after each pass (arpeggio_fx.cu:90-93)
               best = de;
               bdn = dn ^ fb;
@@ -691,9 +706,13 @@ static cudaError_t launch_widths(Widths& wd, Kern kern, size_t key, Smem smem, c
   if (warps > 0)
     for (wi = 4; wi > 0 && ((1 << wi) > warps || nb[wi] == 0);) --wi;
   while (wi > 0 && (1 << (wi - 1)) * A >= a.R) --wi;
-  // one anneal per warp: blocks of four warps while every block finds an SM of its own (one 32-user frame: 44 us
-  // against 46 with eight; 64 frames: 69 against 63)
-  if (A == 1 && warps <= 0 && wi == 3 && (long long)a.B * ((a.R + 3) / 4) <= sms) wi = 2;
+  // one anneal per warp, every block resident at once: blocks of four warps where they leave fewer warps on the fullest SM
+  // than blocks of eight (one 32-user frame: 44 us against 46 with eight, 37 26-user frames, 33 anneals a use, in
+  // the chain of map, anneal and readout: 70 against 75; 64 32-user frames: 69 against 63 with eight)
+  if (A == 1 && warps <= 0 && wi == 3) {
+    const auto fullest = [&](int W) { return (a.B * (long long)((a.R + W - 1) / W) + sms - 1) / sms; };
+    if (fullest(8) <= nb[3] && 4 * fullest(4) < 8 * fullest(8) && nb[2]) wi = 2;
+  }
   if (nb[wi] == 0) return cudaErrorInvalidConfiguration;
   const int W = 1 << wi;
   // small batches: each problem's anneals over several blocks, as many as make the call shortest in anneals one after

@@ -466,9 +466,17 @@ template <int P>
 __host__ __device__ inline size_t sched_bytes(int L) {
   return L <= kMaxSched ? (size_t)((L + 4 * P - 1) / (4 * P) * 4 * P * 8 + 15) / 16 * 16 : 0;
 }
-template <int LN, int C, int P>
+// Whether a kernel keeps stored thresholds.  The engine's numbers have none; and where six copies above 96 coordinates
+// fill the GPU (MB > 1) they are left out: 48 KB for eight warps beside 64 KB of G leave one block an SM instead of two,
+// and the energies of a fixed-point problem whose largest coefficient is in G are beyond 32 bits there (1500 60-user uses
+// of six copies, 8 anneals each: 2535 us with them, 1963 without; the kernel before the several-anneals ones 2304).
+template <int LN, int C, int P, Rule RULE, int MB>
+__host__ __device__ constexpr bool stored() {
+  return RULE != kEngine && !(LN == 32 && C == 4 && P == 6 && MB > 1);
+}
+template <int LN, int C, int P, bool STORED = true>
 inline size_t smem_bytes(int L, int W) {
-  const size_t s = g_bytes<LN, C>() + sched_bytes<P>(L) + (size_t)W * P * C * 256;
+  const size_t s = g_bytes<LN, C>() + sched_bytes<P>(L) + (STORED ? (size_t)W * P * C * 256 : 0);
   const size_t rows = ((size_t)(C - 1) * LN + 33) * LN * C * 4;
   return s > rows ? s : rows;
 }
@@ -476,7 +484,7 @@ inline size_t smem_bytes(int L, int W) {
 // One problem b of a block: G and the schedule staged in shared memory, then the block's anneals.  Called by the
 // per-launch kernel (one problem per block) and by the persistent mixed-size kernel (problems taken from a work
 // counter, one after another).
-template <int LN, int C, int P, Rule RULE>
+template <int LN, int C, int P, Rule RULE, bool STORED = true>
 __device__ __forceinline__ void problem(const DDParams& a, const PhiloxKeys& K, const int b, const int bs) {
   constexpr int DP = LN * C;
   constexpr bool CHORD = RULE == kChord || RULE == kEngine, WARM = RULE == kWarm;
@@ -625,7 +633,7 @@ __device__ __forceinline__ void problem(const DDParams& a, const PhiloxKeys& K, 
       }
     }
   }
-  if constexpr (RULE == kEngine) {
+  if constexpr (!STORED) {
     run<LN, C, P, RULE, true>(a, K, b, bs, Gs, sched, words, s_perm, inst, Rb);
   } else {
     // |psi| <= |h| + (2 P D + 2) max |G| at any state; a pass adds at most D of them and the energy of any state
@@ -654,7 +662,7 @@ __global__ void __launch_bounds__(max_threads<LN, C>(), MB) k_anneal_grp(const D
   const int split = a.split, b = blockIdx.x / split, bs = blockIdx.x - b * split;
   pdl_trigger();
   pdl_wait();
-  problem<LN, C, P, RULE>(a, *reinterpret_cast<const PhiloxKeys*>(a.rk0), b, bs);
+  problem<LN, C, P, RULE, stored<LN, C, P, RULE, MB>()>(a, *reinterpret_cast<const PhiloxKeys*>(a.rk0), b, bs);
 }
 
 // A kernel's resident blocks per SM at each block width (1, 2, 4, 8, 16 warps) for one shared-memory layout, and the
@@ -737,7 +745,7 @@ template <int LN, int C, int P, Rule RULE, int MB = min_blocks<LN, C>()>
 static cudaError_t launch(const DDParams& a, int warps, cudaStream_t st) {
   static Widths wd;
   return launch_widths<32 / LN, max_threads<LN, C>() / 32>(
-      wd, k_anneal_grp<LN, C, P, RULE, MB>, sched_bytes<P>(a.L), [&](int W) { return smem_bytes<LN, C, P>(a.L, W); }, a,
+      wd, k_anneal_grp<LN, C, P, RULE, MB>, sched_bytes<P>(a.L), [&](int W) { return smem_bytes<LN, C, P, stored<LN, C, P, RULE, MB>()>(a.L, W); }, a,
       warps, st);
 }
 

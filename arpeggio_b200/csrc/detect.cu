@@ -114,8 +114,10 @@ __device__ __forceinline__ float row_dot(const float (&x)[TB], const float (&y)[
 // Gram on the tensor cores: digit planes of one row chunk (CH rows of H) in the canonical K-major no-swizzle
 // layout of 8-bit operands -- core matrices of 8 rows (coordinates, the uses' one after another) x 16 bytes (rows of
 // H), LBO = 128 B between neighbours along K, SBO = (CH / 16) 128 B between 8-coordinate groups; one MMA consumes K = 32
-// (two core matrices).  MP = the MMA's M and N: 64 for Dp <= 64, else 128; with several uses the blocks off the
-// diagonal are computed and ignored.
+// (two core matrices).  MP = the MMA's M: 64 for Dp <= 64, else 128, rows above the uses' coordinates unset and their
+// results unread; N = U Dp, and the four accumulators take 4 U Dp TMEM columns (64 for one use of up to 16 coordinates,
+// so that no small block waits for another's release); with several uses the blocks off the diagonal are computed and
+// ignored.
 template <int Dp>
 __host__ __device__ constexpr int kMmaM() { return Dp <= 64 ? 64 : 128; }
 template <int Dp>
@@ -152,8 +154,13 @@ struct MapShape {
   static constexpr int Dp = 16 * TB, U = U_, RB = RB_, TPU = 16 * (Dp / RB);
   static constexpr int NT = U * TPU, HP = Dp + 4, QP = Dp + 4, CH = kChunkRows<Dp>(), MP = kMmaM<Dp>();
   static constexpr int PB = kPlaneBytes<Dp>(), WPU = TPU / 32;  // bytes of a digit plane, warps per use
-  static constexpr uint32_t NCOL = 4 * MP;                      // four class accumulators
+  static constexpr int NN = U * Dp;                             // the MMA's N: the uses' coordinates
+  static constexpr uint32_t NCOL = 4 * NN;                      // four class accumulators
   static constexpr int kFront = PB > U * Dp * QP ? PB : U * Dp * QP;  // floats: four digit planes, later Q
+  // The two-wide multiply-add has the longer latency: it is for the tall tiles, bound by issue; the low ones of small
+  // batches, bound by the chain of pivots, take the scalar one (one 32-user use 30.1 -> 29.4 thousand cycles, one 8-user
+  // use 11.8 -> 11.4, and one row a thread 11.0).
+  static constexpr bool WIDE2 = RB > 4 || U > 1;
   // resident blocks the registers are bounded for: 96 a thread at 64 coordinates, 128 at 128
   static constexpr int MB = TB == 8 ? 2 : TB == 4 && RB == 8 ? 5 : 3;
   static constexpr size_t smem() {
@@ -165,7 +172,8 @@ template <int TB, int RB_, int U_>
 __global__ void __launch_bounds__(MapShape<TB, RB_, U_>::NT, MapShape<TB, RB_, U_>::MB) k_map_dd(const MapParams a) {
   using S = MapShape<TB, RB_, U_>;
   constexpr int Dp = S::Dp, U = S::U, RB = S::RB, TPU = S::TPU, NT = S::NT, HP = S::HP, QP = S::QP, CH = S::CH;
-  constexpr int MP = S::MP, KG = CH / 16, PB = S::PB, WPU = S::WPU, NP = RB / 2;
+  constexpr int MP = S::MP, KG = CH / 16, PB = S::PB, WPU = S::WPU, NP = (RB + 1) / 2;
+  constexpr int NN = S::NN;
   constexpr uint32_t NCOL = S::NCOL;
   extern __shared__ __align__(128) float smap[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -231,7 +239,7 @@ __global__ void __launch_bounds__(MapShape<TB, RB_, U_>::NT, MapShape<TB, RB_, U
     set_scale(mx);
   }
   float gacc = 0.0f;
-  constexpr uint32_t IDESC = umma::idesc_s8(MP, MP);
+  constexpr uint32_t IDESC = umma::idesc_s8(MP, NN);
   const uint32_t pbase = umma::su32(planes);
   int nchunk = 0;
   for (int r0 = 0; r0 < NR2; r0 += CH, ++nchunk) {
@@ -315,7 +323,7 @@ __global__ void __launch_bounds__(MapShape<TB, RB_, U_>::NT, MapShape<TB, RB_, U
           const uint64_t bd = umma::sdesc(pbase + kPairB[q] * PB + ks * 256, 128, KG * 128);
           // the first product of each class in the first chunk starts its accumulator
           const bool first = nchunk == 0 && ks == 0 && (q == 0 || q == 1 || q == 3 || q == 6);
-          umma::mma_s8(tmem + (uint32_t)(kPairC[q] * MP), ad, bd, IDESC, first ? 0u : 1u);
+          umma::mma_s8(tmem + (uint32_t)(kPairC[q] * NN), ad, bd, IDESC, first ? 0u : 1u);
         }
       }
       umma::commit(&mma_bar);
@@ -354,9 +362,9 @@ __global__ void __launch_bounds__(MapShape<TB, RB_, U_>::NT, MapShape<TB, RB_, U
       uint32_t v6[8], v5[8], v4[8], v3[8];
       const uint32_t ta = tmem + ((uint32_t)(wq * 32) << 16) + (uint32_t)(eu * Dp + c0);
       umma::tmem_ld8_nowait(ta, v6);
-      umma::tmem_ld8_nowait(ta + MP, v5);
-      umma::tmem_ld8_nowait(ta + 2 * MP, v4);
-      umma::tmem_ld8_nowait(ta + 3 * MP, v3);
+      umma::tmem_ld8_nowait(ta + NN, v5);
+      umma::tmem_ld8_nowait(ta + 2 * NN, v4);
+      umma::tmem_ld8_nowait(ta + 3 * NN, v3);
       umma::tmem_wait_ld();
       if (valid) {
         float qv[8];
@@ -383,6 +391,11 @@ __global__ void __launch_bounds__(MapShape<TB, RB_, U_>::NT, MapShape<TB, RB_, U
     float q[2][TB];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
+      if (2 * i + h >= RB) {  // one row a thread: the pair's other half is unused
+#pragma unroll
+        for (int j = 0; j < TB; ++j) q[h][j] = 0.0f;
+        continue;
+      }
       lds_vec<TB>(Qs + (ty * RB + 2 * i + h) * QP + tx * TB, q[h]);
 #pragma unroll
       for (int j = 0; j < TB; ++j) {
@@ -425,7 +438,14 @@ __global__ void __launch_bounds__(MapShape<TB, RB_, U_>::NT, MapShape<TB, RB_, U
         }
         if (colown) {
 #pragma unroll
-          for (int i = 0; i < NP; ++i) reinterpret_cast<uint64_t*>(ck + buf + ty * RB)[i] = A[i][kc];
+          for (int i = 0; i < NP; ++i) {
+            if constexpr (RB > 1) {
+              reinterpret_cast<uint64_t*>(ck + buf + ty * RB)[i] = A[i][kc];
+            } else {
+              float t;
+              unpack2(A[i][kc], ck[buf + ty], t);
+            }
+          }
         }
         __syncthreads();
         const float inv = __frcp_rn(rk[buf + k]);
@@ -437,14 +457,27 @@ __global__ void __launch_bounds__(MapShape<TB, RB_, U_>::NT, MapShape<TB, RB_, U
           float f[RB];
           lds_vec<RB>(ck + buf + ty * RB, f);
 #pragma unroll
-          for (int i = 0; i < NP; ++i) nf[i] = mul2(pack2(f[2 * i], f[2 * i + 1]), ninv);
+          for (int i = 0; i < NP; ++i) {
+            const float f1 = 2 * i + 1 < RB ? f[2 * i + 1] : 0.0f;
+            nf[i] = S::WIDE2 ? mul2(pack2(f[2 * i], f1), ninv)
+                             : pack2(__fmul_rn(f[2 * i], -inv), __fmul_rn(f1, -inv));
+          }
         }
 #pragma unroll
         for (int j = 0; j < TB; ++j) rd[j] = pack2(rj[j], rj[j]);
 #pragma unroll
         for (int i = 0; i < NP; ++i)
 #pragma unroll
-          for (int j = 0; j < TB; ++j) A[i][j] = fma2(nf[i], rd[j], A[i][j]);
+          for (int j = 0; j < TB; ++j) {
+            if constexpr (S::WIDE2) {
+              A[i][j] = fma2(nf[i], rd[j], A[i][j]);
+            } else {
+              float n0, n1, a0, a1;
+              unpack2(nf[i], n0, n1);
+              unpack2(A[i][j], a0, a1);
+              A[i][j] = pack2(__fmaf_rn(n0, rj[j], a0), __fmaf_rn(n1, rj[j], a1));
+            }
+          }
         auto set = [&](uint64_t& v, float x) {  // the pair's half of row kr
           float lo, hi;
           unpack2(v, lo, hi);
@@ -942,7 +975,7 @@ cudaError_t map_dispatch(const MapParams& a, cudaStream_t st) {
   if (D > 64) return launch_map<8, 8, 1>(a, st);
   if (D > 32) return small ? launch_map<4, 4, 1>(a, st) : launch_map<4, 8, 1>(a, st);
   if (D > 16) return small ? launch_map<2, 2, 1>(a, st) : launch_map<2, 4, 2>(a, st);
-  return small ? launch_map<1, 2, 1>(a, st) : launch_map<1, 4, 4>(a, st);
+  return small ? launch_map<1, 1, 1>(a, st) : launch_map<1, 4, 4>(a, st);
 }
 
 static size_t readout_smem(int D, int NR2, int R, bool soft = false) {

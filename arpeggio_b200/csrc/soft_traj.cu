@@ -21,6 +21,9 @@
 // of flips among the chains) instead of voted on.  What bounds it is the rows of J: a flip reads one, two wavefronts
 // of shared memory at 64 spins, and they keep its pipe 71 % busy (issue slots 60 %; 1990 instructions per step of four
 // chains, 1826 per step of one before).  4096 16-user uses, 16 chains x 256 steps: 32.5 -> 11.6 ms.
+// With few chains a problem's blocks are what is resident, so J takes a row per spin and columns to the next multiple of
+// LN only (36 KB at 96 spins), and where it is large more warps than the chains need help to stage it: 1400 24-user
+// uses of one 64-step chain 2796 us with 64 KB rounded up to whole slots and one warp, 1927 now; of five 3171 and 2280.
 // The reference draws its chains' start and tests from torch.rand; this sampler draws them from Philox counters of
 // its own (start: word 0 of (2^32 - 1, i, r, inst), spin +1 iff >= 2^31), so its trajectories are its own while the
 // rule, the visited-state bookkeeping and the LLR formation are the reference's.
@@ -70,30 +73,65 @@ struct SoftMap {
   static constexpr int A = 32 / LN, C = QAM ? 2 * CD : CD, DP = LN * C, NB = QAM ? 2 : 1;
 };
 
+// A lane's C entries of a row lie side by side in planes of four slots (one 16-byte load), then two: position of slot c of
+// group lane ln.
+template <int LN, int C>
+__device__ __forceinline__ int row_pos(int c, int ln) {
+  return c < (C & ~3) ? (c >> 2) * 4 * LN + ln * 4 + (c & 3) : (C & ~3) * LN + ln * 2 + (c & 1);
+}
+
 template <int LN, int CD, bool QAM>
 __global__ void __launch_bounds__(32 * kSoftWarps) k_traj_soft(const SoftParams a) {
   using M = SoftMap<LN, CD, QAM>;
   constexpr int A = M::A, C = M::C, DP = M::DP, NB = M::NB;
   extern __shared__ __align__(16) float sms[];
   const int N = a.N, D = a.D, S = a.S, R = a.R;
-  const int b = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5, W = blockDim.x >> 5;
+  // the first W warps run chains; a block of few chains has more, which help to stage J
+  const int b = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5, BW = blockDim.x >> 5;
+  const int W = min(BW, (R + A - 1) / A);
   const int ln = lane & (LN - 1), grp = lane / LN, li = LN - 1 - ln;  // the first coordinate on the highest lane
   const uint32_t gmask = (LN == 32 ? ARP_FULL : (1u << (LN & 31)) - 1u) << (grp * LN);
-  float* Js = sms;                          // DP x DP, rows and columns in slot order, a lane's C entries by fours
-  float* ws = Js + DP * DP + wid * 4 * C * 32;  // the warp's scratch
-  float* redm = Js + DP * DP + W * 4 * C * 32;  // W x 2 x (CD NB) x LN: minima by group lane
+  float* Js = sms;                          // N x DP: the spins' rows, columns by row_pos
+  float* ws = Js + N * DP + wid * 4 * C * 32;  // the warp's scratch
+  float* redm = Js + N * DP + W * 4 * C * 32;  // W x 2 x (CD NB) x LN: minima by group lane
   float* redb = redm + W * 2 * CD * NB * LN;  // W x 3: best d, step, chain
   uint32_t* redS = reinterpret_cast<uint32_t*>(redb + kSoftWarps * 3);  // W x LN: best spins
   // spin of slot c, group coordinate i
   auto spin = [&](int c, int i) { return QAM && c >= CD ? D + (c - CD) * LN + i : c * LN + i; };
   auto inside = [&](int c, int i) { return (QAM && c >= CD ? c - CD : c) * LN + i < D; };
-  for (int x = threadIdx.x; x < DP * DP; x += blockDim.x) {
-    const int rp = x / DP, cp = x - rp * DP;
-    const int rc = rp / LN, ri = rp & (LN - 1), cc = cp / LN, ci = cp & (LN - 1);
-    const float v = inside(rc, ri) && inside(cc, ci)
-                        ? a.J[(size_t)b * N * N + (size_t)spin(rc, ri) * N + spin(cc, ci)]
-                        : 0.0f;
-    Js[rp * DP + (cc >> 2) * 4 * LN + (LN - 1 - ci) * 4 + (cc & 3)] = v;
+  {  // a row per warp, four rows in flight
+    constexpr int CW = (DP + 31) / 32;
+    const float* Jb = a.J + (size_t)b * N * N;
+    int pos[CW];  // place of the row's entry k 32 + lane; beyond the spins, of a column without one (zero)
+#pragma unroll
+    for (int k = 0; k < CW; ++k) {
+      const int x = k * 32 + lane;
+      int c, i;
+      if (x < N) {
+        const int j = QAM && x >= D ? x - D : x;
+        c = j / LN + (QAM && x >= D ? CD : 0);
+        i = j & (LN - 1);
+      } else {  // columns without a spin, in order
+        const int z = x - N, pad = CD * LN - D, h = QAM && z >= pad ? 1 : 0, j = D + z - h * pad;
+        c = j / LN + h * CD;
+        i = j & (LN - 1);
+      }
+      pos[k] = x < DP ? row_pos<LN, C>(c, LN - 1 - i) : 0;
+    }
+#pragma unroll 1
+    for (int r0 = wid; r0 < N; r0 += 4 * BW) {
+      float v[4][CW];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int k = 0; k < CW; ++k)
+          v[u][k] = r0 + u * BW < N && k * 32 + lane < N ? Jb[(size_t)(r0 + u * BW) * N + k * 32 + lane] : 0.0f;
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int k = 0; k < CW; ++k)
+          if (r0 + u * BW < N && k * 32 + lane < DP) Js[(r0 + u * BW) * DP + pos[k]] = v[u][k];
+    }
   }
   __syncthreads();
   const uint32_t inst = a.inst[b];
@@ -120,14 +158,19 @@ __global__ void __launch_bounds__(32 * kSoftWarps) k_traj_soft(const SoftParams 
   int wstep = INT_MAX, wchain = INT_MAX;
   uint32_t wup = 0;
   auto row = [&](int c, int l, float(&g)[C]) {  // row of slot c, group lane l
-    const float* p = Js + (c * LN + LN - 1 - l) * DP + ln * 4;
+    const float* p = Js + spin(c, LN - 1 - l) * DP;
 #pragma unroll
     for (int q = 0; q < C / 4; ++q) {
-      const float4 v = *reinterpret_cast<const float4*>(p + q * 4 * LN);
+      const float4 v = *reinterpret_cast<const float4*>(p + ln * 4 + q * 4 * LN);
       g[4 * q] = v.x;
       g[4 * q + 1] = v.y;
       g[4 * q + 2] = v.z;
       g[4 * q + 3] = v.w;
+    }
+    if constexpr (C & 2) {
+      const float2 v = *reinterpret_cast<const float2*>(p + ln * 2 + (C & ~3) * LN);
+      g[C - 2] = v.x;
+      g[C - 1] = v.y;
     }
   };
   for (int r0 = wid * A; r0 < R; r0 += W * A) {
@@ -228,7 +271,8 @@ __global__ void __launch_bounds__(32 * kSoftWarps) k_traj_soft(const SoftParams 
         const bool su = (up >> c) & 1u;
         const float cfl = su ? -4.0f : 4.0f, s2 = su ? 2.0f : -2.0f;
         for (int t = 0; t < rounds; ++t) {
-          const int l = high_bit(mg);  // -1 without a flip left: lane 31 of the group is read, nothing is changed
+          // -1 without a flip left: the slot's first spin (the group's highest lane) is read, nothing is changed
+          const int l = high_bit(mg);
           const int has = (int)mg;
           mg &= ~(1u << (l & 31));
           // dE0 = 2 s_j (h0_j + u_j - hf_j)
@@ -271,7 +315,7 @@ __global__ void __launch_bounds__(32 * kSoftWarps) k_traj_soft(const SoftParams 
       wup = cup;
     }
   }
-  // ---- the minima and the best over the warp's groups, then over the block's warps
+  // ---- the minima and the best over the warp's groups, then over the chains' warps
 #pragma unroll
   for (int o = LN; o < 32; o <<= 1) {
 #pragma unroll
@@ -289,7 +333,7 @@ __global__ void __launch_bounds__(32 * kSoftWarps) k_traj_soft(const SoftParams 
       wup = ou;
     }
   }
-  if (lane < LN) {
+  if (lane < LN && wid < W) {
 #pragma unroll
     for (int c = 0; c < CD * NB; ++c) {
       redm[((wid * 2 + 0) * CD * NB + c) * LN + lane] = mn0[c];
@@ -297,7 +341,7 @@ __global__ void __launch_bounds__(32 * kSoftWarps) k_traj_soft(const SoftParams 
     }
     redS[wid * LN + lane] = wup;
   }
-  if (lane == 0) {
+  if (lane == 0 && wid < W) {
     redb[wid * 3] = wbest;
     redb[wid * 3 + 1] = __int_as_float(wstep);
     redb[wid * 3 + 2] = __int_as_float(wchain);
@@ -332,15 +376,17 @@ __global__ void __launch_bounds__(32 * kSoftWarps) k_traj_soft(const SoftParams 
 template <int LN, int CD, bool QAM>
 static cudaError_t launch_soft(const SoftParams& a, cudaStream_t st) {
   using M = SoftMap<LN, CD, QAM>;
-  const int W = min(kSoftWarps, (a.R + M::A - 1) / M::A);
-  const size_t smem = 4 * ((size_t)M::DP * M::DP + (size_t)W * 4 * M::C * 32 + (size_t)W * 2 * CD * M::NB * LN +
+  // up to 64 spins the chains' warps stage J alone: more warps would hold registers that other blocks' chains need
+  // (1400 uses of 64 spins, one chain each: 1345 us with one warp, 1547 with two)
+  const int W = min(kSoftWarps, (a.R + M::A - 1) / M::A), stage = a.N <= 64 ? 1 : a.N <= 96 ? 4 : kSoftWarps;
+  const size_t smem = 4 * ((size_t)a.N * M::DP + (size_t)W * 4 * M::C * 32 + (size_t)W * 2 * CD * M::NB * LN +
                            kSoftWarps * 3 + (size_t)W * LN);
   if (smem > 48 * 1024) {
     cudaError_t e =
         cudaFuncSetAttribute(k_traj_soft<LN, CD, QAM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  k_traj_soft<LN, CD, QAM><<<a.B, 32 * W, smem, st>>>(a);
+  k_traj_soft<LN, CD, QAM><<<a.B, 32 * max(W, stage), smem, st>>>(a);
   return cudaGetLastError();
 }
 
@@ -361,8 +407,16 @@ extern "C" int arp_soft_trajectory(const float* J, const float* hf, const float*
   cudaStream_t st = (cudaStream_t)stream;
   cudaError_t e;
   if (M == 16)
-    e = D <= 16 ? launch_soft<8, 2, true>(a, st) : D <= 32 ? launch_soft<8, 4, true>(a, st) : launch_soft<16, 4, true>(a, st);
+    e = D <= 16   ? launch_soft<8, 2, true>(a, st)
+        : D <= 24 ? launch_soft<8, 3, true>(a, st)
+        : D <= 32 ? launch_soft<8, 4, true>(a, st)
+        : D <= 48 ? launch_soft<16, 3, true>(a, st)
+                  : launch_soft<16, 4, true>(a, st);
   else
-    e = D <= 32 ? launch_soft<8, 4, false>(a, st) : D <= 64 ? launch_soft<8, 8, false>(a, st) : launch_soft<16, 8, false>(a, st);
+    e = D <= 32   ? launch_soft<8, 4, false>(a, st)
+        : D <= 48 ? launch_soft<8, 6, false>(a, st)
+        : D <= 64 ? launch_soft<8, 8, false>(a, st)
+        : D <= 96 ? launch_soft<16, 6, false>(a, st)
+                  : launch_soft<16, 8, false>(a, st);
   return e == cudaSuccess ? ARP_OK : ARP_ERR_LAUNCH;
 }

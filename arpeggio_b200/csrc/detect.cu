@@ -18,6 +18,7 @@
 //   candidate r: x = clip(x_q + sum_p s_p) to the constellation; dist = ||y - H x||^2; the first
 //   minimum over the R candidates then the guess x_q; Gray bits per dimension, MSB first.
 #include <cfloat>
+#include <type_traits>
 
 #include "arp_common.cuh"
 #include "arp_internal.h"
@@ -74,6 +75,23 @@ __device__ __forceinline__ void lds_vec(const float* p, float (&v)[TB]) {
   } else {
 #pragma unroll
     for (int i = 0; i < TB; ++i) v[i] = p[i];
+  }
+}
+// V floats of global memory as one load, aligned to its size.
+template <int V>
+__device__ __forceinline__ void ldg_vec(const float* p, float (&v)[V]) {
+  if constexpr (V == 4) {
+    const float4 t = *reinterpret_cast<const float4*>(p);
+    v[0] = t.x;
+    v[1] = t.y;
+    v[2] = t.z;
+    v[3] = t.w;
+  } else if constexpr (V == 2) {
+    const float2 t = *reinterpret_cast<const float2*>(p);
+    v[0] = t.x;
+    v[1] = t.y;
+  } else {
+    v[0] = *p;
   }
 }
 template <int TB>
@@ -161,8 +179,9 @@ struct MapShape {
   // batches, bound by the chain of pivots, take the scalar one (one 32-user use 30.1 -> 29.4 thousand cycles, one 8-user
   // use 11.8 -> 11.4, and one row a thread 11.0).
   static constexpr bool WIDE2 = RB > 4 || U > 1;
-  // resident blocks the registers are bounded for: 96 a thread at 64 coordinates, 128 at 128
-  static constexpr int MB = TB == 8 ? 2 : TB == 4 && RB == 8 ? 5 : 3;
+  // resident blocks the registers are bounded for: 96 a thread at 64 coordinates, 128 at 128, 64 for several uses (72
+  // registers, three blocks instead of four, cost 4000 16-user uses a tenth)
+  static constexpr int MB = TB == 8 ? 2 : TB == 4 && RB == 8 ? 5 : U > 1 ? 4 : 3;
   static constexpr size_t smem() {
     return sizeof(float) * (kFront + U * (CH * HP + 6 * Dp + CH) + NT / 32);
   }
@@ -248,26 +267,31 @@ __global__ void __launch_bounds__(MapShape<TB, RB_, U_>::NT, MapShape<TB, RB_, U
     if (s_abort) break;
     for (int x = ut; x < nr; x += TPU) yc[x] = on ? yb[r0 + x] : 0.0f;
     float mx = 0.0f;
-    if ((D & 3) == 0 && (reinterpret_cast<uintptr_t>(a.H) & 15u) == 0) {  // 16-byte loads, Dp / 4 threads a row
-      constexpr int QR = Dp / 4, RS = TPU / QR;
-      const int q4 = 4 * (ut & (QR - 1));
-      const bool in = on && q4 < D;
+    // the widest loads the rows' alignment allows, Dp / V threads a row, four in flight (an odd number of users has rows
+    // aligned to 8 bytes: the map of 4000 29-user uses by 4-byte loads, two in flight, 317 us, by these 240)
+    auto stage = [&](auto width) {
+      constexpr int V = decltype(width)::value, QR = Dp / V, RS = TPU / QR;
+      const int q = V * (ut & (QR - 1));
+      const bool in = on && q < D;
 #pragma unroll 4
       for (int r = ut / QR; r < nr; r += RS) {
-        const float4 v = in ? *reinterpret_cast<const float4*>(Hb + (size_t)(r0 + r) * D + q4)
-                            : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        *reinterpret_cast<float4*>(Hc + r * HP + q4) = v;
-        mx = fmaxf(fmaxf(mx, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
+        float v[V];
+        if (in)
+          ldg_vec<V>(Hb + (size_t)(r0 + r) * D + q, v);
+        else
+#pragma unroll
+          for (int i = 0; i < V; ++i) v[i] = 0.0f;
+        sts_vec<V>(Hc + r * HP + q, v);
+#pragma unroll
+        for (int i = 0; i < V; ++i) mx = fmaxf(mx, fabsf(v[i]));
       }
-    } else {
-#pragma unroll 2
-      for (int x = ut; x < nr * Dp; x += TPU) {
-        const int r = x / Dp, j = x - r * Dp;
-        const float v = on && j < D ? Hb[(size_t)(r0 + r) * D + j] : 0.0f;
-        Hc[r * HP + j] = v;
-        mx = fmaxf(mx, fabsf(v));
-      }
-    }
+    };
+    if ((D & 3) == 0 && (reinterpret_cast<uintptr_t>(a.H) & 15u) == 0)
+      stage(std::integral_constant<int, 4>());
+    else if ((D & 1) == 0 && (reinterpret_cast<uintptr_t>(a.H) & 7u) == 0)
+      stage(std::integral_constant<int, 2>());
+    else
+      stage(std::integral_constant<int, 1>());
     if (one_chunk)
       set_scale(mx);  // its barriers also publish the staged rows
     else

@@ -34,9 +34,11 @@
 // kMaxSched passes (every fixed-point problem of to_fixed, where |G|, |h| <= 4096) run with 32-bit energies and the
 // stored thresholds; the others run the same scan with 64-bit energies and one Philox block per pass (Wide).
 #pragma once
+#include <array>
 #include <climits>
 #include <mutex>
 #include <type_traits>
+#include <unordered_map>
 
 #include "arp_common.cuh"
 #include "arp_internal.h"
@@ -665,13 +667,15 @@ __global__ void __launch_bounds__(max_threads<LN, C>(), MB) k_anneal_grp(const D
   problem<LN, C, P, RULE, stored<LN, C, P, RULE, MB>()>(a, *reinterpret_cast<const PhiloxKeys*>(a.rk0), b, bs);
 }
 
-// A kernel's resident blocks per SM at each block width (1, 2, 4, 8, 16 warps) for one shared-memory layout, and the
-// dynamic shared memory it may use, per device.
+// Per device: a kernel's resident blocks per SM at each block width (1, 2, 4, 8, 16 warps) for every shared-memory layout
+// it was launched with (one per staged schedule length: at most 130), and the dynamic shared memory it may use.  A launch
+// with a layout met before asks the runtime nothing.
 struct Widths {
   std::mutex mu;
   struct Dev {
-    size_t key = 0, limit = 48 * 1024;
-    int nb[5] = {}, sms = 0;
+    size_t limit = 48 * 1024;
+    int sms = 0;
+    std::unordered_map<size_t, std::array<int, 5>> nb;
   } dev[kMaxDevices];
 };
 constexpr size_t kMaxDynamic = 226 * 1024;
@@ -691,20 +695,21 @@ static cudaError_t launch_widths(Widths& wd, Kern kern, size_t key, Smem smem, c
     d.limit = bytes;
     return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   };
-  if (d.key != key + 1) {
+  auto known = d.nb.find(key);
+  if (known == d.nb.end()) {
     if ((e = cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
     const size_t was = d.limit;
     if ((e = limit(kMaxDynamic)) != cudaSuccess) return e;
+    std::array<int, 5> n{};
     for (int i = 0; i < 5; ++i) {
-      d.nb[i] = 0;
       if ((1 << i) > WMAX || smem(1 << i) > kMaxDynamic) continue;
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.nb[i], kern, 32 << i, smem(1 << i));
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n[i], kern, 32 << i, smem(1 << i));
       if (e != cudaSuccess) return e;
     }
     if ((e = limit(was)) != cudaSuccess) return e;
-    d.key = key + 1;
+    known = d.nb.emplace(key, n).first;
   }
-  const int(&nb)[5] = d.nb;
+  const std::array<int, 5>& nb = known->second;
   const int sms = d.sms;
   // the width with the most resident warps per SM (ties: the wider block, which stages G fewer times per anneal),
   // or the caller's; no wider than the problem's anneals need
@@ -745,8 +750,8 @@ template <int LN, int C, int P, Rule RULE, int MB = min_blocks<LN, C>()>
 static cudaError_t launch(const DDParams& a, int warps, cudaStream_t st) {
   static Widths wd;
   return launch_widths<32 / LN, max_threads<LN, C>() / 32>(
-      wd, k_anneal_grp<LN, C, P, RULE, MB>, sched_bytes<P>(a.L), [&](int W) { return smem_bytes<LN, C, P, stored<LN, C, P, RULE, MB>()>(a.L, W); }, a,
-      warps, st);
+      wd, k_anneal_grp<LN, C, P, RULE, MB>, sched_bytes<P>(a.L),
+      [&](int W) { return smem_bytes<LN, C, P, stored<LN, C, P, RULE, MB>()>(a.L, W); }, a, warps, st);
 }
 
 // How many anneals share a warp is a matter of how many there are: A per warp need A times as many to fill the GPU.

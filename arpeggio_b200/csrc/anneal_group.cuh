@@ -494,7 +494,7 @@ __device__ __forceinline__ void problem(const DDParams& a, const PhiloxKeys& K, 
   int32_t* Gs = reinterpret_cast<int32_t*>(smem);
   __shared__ int s_bad, s_wt;
   __shared__ uint32_t s_mg, s_mh;
-  __shared__ uint8_t s_perm[WARM ? 128 : 1], s_inv[WARM ? 128 : 1];
+  __shared__ uint8_t s_perm[WARM ? 128 : 1];
   const int D = a.D, L = a.L, R = a.R, bt = blockDim.x;
   int2* sched = reinterpret_cast<int2*>(smem + g_bytes<LN, C>());
   uint32_t* words = reinterpret_cast<uint32_t*>(smem + g_bytes<LN, C>() + sched_bytes<P>(L));
@@ -510,10 +510,11 @@ __device__ __forceinline__ void problem(const DDParams& a, const PhiloxKeys& K, 
   const int32_t* Gg = reinterpret_cast<const int32_t*>(a.Gt) + (size_t)b * D * D;
   uint32_t mg = 0, mh = 0;  // largest |G|, |h| (as unsigned: |INT_MIN| = 2^31)
   bool bad = false;
-  // G by 16-byte loads, eight in flight per thread; a matrix that is not 16-byte aligned, or D no multiple of 4, by
-  // 4-byte loads.  One anneal per warp (small batches, whose instructions come cold from L2 in every frame) takes a
-  // loop of less code instead, a row per warp: 1.5 us less for a 32-user frame than the unrolled one
-  const bool vec = LN < 32 && (D & 3) == 0 && (reinterpret_cast<uintptr_t>(Gg) & 15u) == 0;
+  // G by 16-byte loads, eight in flight per thread.  By 4-byte loads, a row per warp, where the matrix is not 16-byte aligned
+  // or D no multiple of 4 (an odd number of users); for one anneal per warp (small batches, whose instructions come cold
+  // from L2 in every frame: less code, 1.5 us less for a 32-user frame than the unrolled loop); and for a scan order, where
+  // a lane gathers its columns of each row.
+  const bool vec = !WARM && LN < 32 && (D & 3) == 0 && (reinterpret_cast<uintptr_t>(Gg) & 15u) == 0;
   const int D4 = D >> 2, nv = vec ? D * D4 : 0;
   int4 v[8];
   auto fetch = [&](int x0) {
@@ -526,41 +527,20 @@ __device__ __forceinline__ void problem(const DDParams& a, const PhiloxKeys& K, 
   const int x1 = threadIdx.x;
   const int32_t h1 = x1 < D ? hg[x1] : 0, t1 = x1 < L ? Tg[x1] : 0, c1 = (CHORD && cg && x1 < L) ? cg[x1] : 0;
   const uint32_t inst = a.inst ? a.inst[b] : a.inst0 + (uint32_t)b;
-  bool order = true;  // every thread's: perm is an order of 0..D-1
   if constexpr (WARM) {
-    // position j' of the scan holds coordinate perm[j']: G goes into that order by the inverse, h is gathered
+    // position j' of the scan holds coordinate perm[j']: G and h are gathered into that order
     for (int x = threadIdx.x; x < D; x += bt) {
       const uint8_t pv = a.perm[(size_t)b * D + x];
       bad |= pv >= D;  // reported as ARP_ERR_RANGE, never dereferenced
       s_perm[x] = pv < D ? pv : 0;
-      if (pv < D) s_inv[pv] = (uint8_t)x;
     }
-    __syncthreads();
-    bool off = bad;
-    for (int x = threadIdx.x; x < D; x += bt) off |= s_inv[s_perm[x]] != x;
-    order = !__syncthreads_or(off);
-  } else {
-    __syncthreads();
   }
-  auto put = [&](int j, int i, int32_t g) {  // G[j][i] into its place (WARM: in the scan order)
-    if constexpr (WARM) {
-      j = s_inv[j];
-      i = s_inv[i];
-    }
+  __syncthreads();
+  auto put = [&](int j, int i, int32_t g) {  // entry (j, i) into its place
     mg = max(mg, (uint32_t)abs(g));
     Gs[j * DP + row_pos<LN, C>(i / LN, LN - 1 - (i & (LN - 1)))] = g;
   };
-  if (WARM && !order) {
-    // repeated entries: no inverse (s_inv has places that were never written), so G is gathered, entry by entry
-#pragma unroll 1
-    for (int x = threadIdx.x; x < D * D; x += bt) {
-      const int j = x / D, i = x - j * D;
-      const int32_t g = Gg[(int)s_perm[j] * D + s_perm[i]];
-      mg = max(mg, (uint32_t)abs(g));
-      Gs[j * DP + row_pos<LN, C>(i / LN, LN - 1 - (i & (LN - 1)))] = g;
-    }
-  }
-  for (int x0 = order ? (int)threadIdx.x : nv; x0 < nv; x0 += 8 * bt) {
+  for (int x0 = threadIdx.x; x0 < nv; x0 += 8 * bt) {
     if (x0 != (int)threadIdx.x) fetch(x0);
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
@@ -573,24 +553,27 @@ __device__ __forceinline__ void problem(const DDParams& a, const PhiloxKeys& K, 
       put(j, i + 3, v[u].w);
     }
   }
-  if constexpr (LN == 32) {
+  if (WARM || LN == 32 || !vec) {  // a row per warp, four rows in flight
+    constexpr int CW = (DP + 31) / 32;
     const int lane = threadIdx.x & 31, W = bt >> 5;
+    int col[CW];
+#pragma unroll
+    for (int c = 0; c < CW; ++c) col[c] = WARM && c * 32 + lane < D ? s_perm[c * 32 + lane] : c * 32 + lane;
 #pragma unroll 1
-    for (int j0 = order ? (int)threadIdx.x >> 5 : D; j0 < D; j0 += 4 * W) {
-      int32_t g[4][C];
+    for (int j0 = threadIdx.x >> 5; j0 < D; j0 += 4 * W) {
+      int32_t g[4][CW];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int j = j0 + u * W, row = (WARM && j < D ? s_perm[j] : j) * D;
+#pragma unroll
+        for (int c = 0; c < CW; ++c) g[u][c] = (j < D && c * 32 + lane < D) ? Gg[row + col[c]] : 0;
+      }
 #pragma unroll
       for (int u = 0; u < 4; ++u)
 #pragma unroll
-        for (int c = 0; c < C; ++c)
-          g[u][c] = (j0 + u * W < D && c * 32 + lane < D) ? Gg[(j0 + u * W) * D + c * 32 + lane] : 0;
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int c = 0; c < C; ++c)
+        for (int c = 0; c < CW; ++c)
           if (j0 + u * W < D && c * 32 + lane < D) put(j0 + u * W, c * 32 + lane, g[u][c]);
     }
-  } else if (!vec && order) {
-    for (int x = threadIdx.x; x < D * D; x += bt) put(x / D, x % D, Gg[x]);
   }
   for (int x = threadIdx.x; x < D * (DP - D); x += bt) {  // padding columns
     const int j = x / (DP - D), i = D + x - j * (DP - D);

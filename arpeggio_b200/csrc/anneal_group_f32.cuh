@@ -137,6 +137,7 @@ __global__ void __launch_bounds__(grp::max_threads<LN, C>(), MB) k_anneal_f32(co
 #pragma unroll
       for (int p = 0; p < P; ++p) d += (dn >> (p * C + c)) & 1u;
       const float mc = ((vm >> c) & 1u) ? (float)(P - 2 * d) : 0.0f;
+      if (!__any_sync(ARP_FULL, mc != 0.0f)) continue;  // as in the integer kernel
 #pragma unroll 2
       for (int i = 0; i < LN; ++i) {
         if (c * LN + i >= D) break;

@@ -415,7 +415,7 @@ __device__ __forceinline__ void run(const DDParams& a, const PhiloxKeys& K, cons
             if (a.out_n1) n1 += (__ballot_sync(ARP_FULL, (fb >> (p * C)) != 0) & gmask) != 0;
           }
           if (SPREAD || any) {
-            if constexpr (LN == 32 && !SPREAD) {
+            if constexpr (LN == 32 && !SPREAD && !WIDE) {
               de += __reduce_add_sync(ARP_FULL, e);
             } else if constexpr (!SPREAD) {
 #pragma unroll
@@ -705,12 +705,12 @@ static cudaError_t launch_widths(Widths& wd, Kern kern, size_t key, Smem smem, c
   if (warps > 0)
     for (wi = 4; wi > 0 && ((1 << wi) > warps || nb[wi] == 0);) --wi;
   while (wi > 0 && (1 << (wi - 1)) * A >= a.R) --wi;
-  // one anneal per warp, every block resident at once: blocks of four warps where they leave fewer warps on the fullest SM
-  // than blocks of eight (one 32-user frame: 44 us against 46 with eight, 37 26-user frames, 33 anneals a use, in
-  // the chain of map, anneal and readout: 70 against 75; 64 32-user frames: 69 against 63 with eight)
-  if (A == 1 && warps <= 0 && wi == 3) {
+  // one anneal per warp, every block resident at once: blocks of eight warps, or of four where those leave fewer warps on
+  // the fullest SM (one 32-user frame: 44 us against 46 with eight; 37 26-user frames, 33 anneals a use, in the chain
+  // of map, anneal and readout: 70 against 75; 64 32-user frames: 69 against 63 with eight)
+  if (A == 1 && warps <= 0 && (wi == 2 || wi == 3) && a.R > 4) {
     const auto fullest = [&](int W) { return (a.B * (long long)((a.R + W - 1) / W) + sms - 1) / sms; };
-    if (fullest(8) <= nb[3] && 4 * fullest(4) < 8 * fullest(8) && nb[2]) wi = 2;
+    if (fullest(8) <= nb[3] && fullest(4) <= nb[2]) wi = 4 * fullest(4) < 8 * fullest(8) ? 2 : 3;
   }
   if (nb[wi] == 0) return cudaErrorInvalidConfiguration;
   const int W = 1 << wi;
@@ -746,8 +746,10 @@ static cudaError_t launch(const DDParams& a, int warps, cudaStream_t st) {
 // which half the full mapping's anneals per warp win, by coordinates.  32 anneals a use, one / two / four per warp at
 // 64 coordinates: 64 uses 63 / 83 / 126 us, 148 uses 121 / 108 / 143, 600 uses 387 / 296 / 308, 1200 uses
 // 727 / 522 / 512; one / two / four at 32: 156 uses 56 / 54 / 63, 312 uses 93 / 75 / 75, 625 uses 184 / 147 / 121;
-// two / four / eight at 16: 156 uses 31 / 35 / 47, 625 uses 84 / 65 / 68, 1250 uses 133 / 106 / 103.
-constexpr long long kLatWarps = 148LL * 16, kOnePerWarp = 148LL * 32;
+// two / four / eight at 16: 156 uses 31 / 35 / 47, 625 uses 84 / 65 / 68, 1250 uses 133 / 106 / 103.  Above 16 coordinates one
+// per warp keeps its lead into a short second wave (37 warps a SM for 32): 76 and 83 14-user uses of 64 anneals in the
+// chain of map, anneal and readout 74 -> 67 and 79 -> 78 us, 120 21-user uses of 33 104 -> 93.
+constexpr long long kLatWarps = 148LL * 16, kOnePerWarp = 148LL * 37;
 constexpr long long kMid16 = 30000, kMid32 = 10000, kMid64 = 148LL * 32 * 8;
 
 // The mapping (LN lanes per anneal, C coordinates per lane) for D coordinates.  P = 6 keeps four coordinates a lane
@@ -767,15 +769,19 @@ static cudaError_t dispatch(const DDParams& a, int warps, cudaStream_t st) {
   // 1200 -> 1060 us, first accept 1510 -> 1365; below 16 a use there are too few warps beside 64 KB of G.
   const bool waste = (a.R + 15) / 16 * 128 > a.R * 9;
   const bool start = RULE == kChord && w8 <= kLatWarps * 5 / 4;  // just above one per warp's first wave: 224 -> 207 us
+  // Per-problem counts, most of them a few anneals in blocks of a few warps: the two-per-warp kernels of 128 coordinates,
+  // bound for blocks of 16 warps, keep two of them an SM, one per warp four (3000 53-user uses, 16 anneals, easy ones 4:
+  // 2667 -> 2420 us; 64-user ones 2705 -> 2440).  Up to 96 coordinates two per warp stay ahead (1790 against 1830).
+  const bool counted = RULE == kWarm && a.ra && D > 96;
   if constexpr (RULE != kEngine && P < 6)
-    if (D > 64 && w8 > kLatWarps / 2 && (w8 <= kLatWarps || ragged || waste || start))
+    if (D > 64 && w8 > kLatWarps / 2 && (w8 <= kLatWarps || ragged || waste || start || counted))
       return D <= 96 ? launch<32, 3, P, RULE>(a, warps, st) : launch<32, 4, P, RULE>(a, warps, st);
   if (RULE != kEngine && w8 <= (D > 64 ? kLatWarps / 2 : kLatWarps))
     return D <= 32   ? launch<32, 1, P, RULE, 1>(a, warps, st)
            : D <= 64 ? launch<32, 2, P, RULE, 1>(a, warps, st)
            : D <= 96 ? launch<32, 3, P, RULE, 1>(a, warps, st)
                      : launch<32, 4, P, RULE, 1>(a, warps, st);
-  if (RULE != kEngine && w8 <= kOnePerWarp && D <= 64)
+  if (RULE != kEngine && w8 <= (D > 16 ? kOnePerWarp : 148LL * 32) && D <= 64)
     return D <= 32 ? launch<32, 1, P, RULE>(a, warps, st) : launch<32, 2, P, RULE>(a, warps, st);
   // few anneals a use leave a wide block's warps without work: the half mapping below 16
   if (D <= 16 && (n <= kMid16 || a.R < 16)) return launch<8, 2, P, RULE>(a, warps, st);

@@ -284,18 +284,20 @@ static cudaError_t dispatch(const DDParams& a, int warps, cudaStream_t st) {
   const int D = a.D;
   const long long n = (long long)a.B * a.R, w8 = (long long)a.B * ((a.R + 7) / 8 * 8);
   // one anneal per warp, as in the integer kernel, for few anneals and for counts that fill their last block of 16 badly
-  // (34000 of 126 coordinates, 33 a use: first accept 2211 -> 2119 us, Chord 1636 -> 1471)
+  // (34000 of 126 coordinates, 33 a use: first accept 2211 -> 2119 us, Chord 1636 -> 1471); into a short second wave (81
+  // uses of 32 anneals in the detector, first accept: 36 users 189 -> 156 us, 63 users 269 -> 230), by Chord above 96
+  // coordinates only; and above 96 coordinates up to 16 anneals a use, which one block of eight two-per-warp warps holds
   const bool waste = (a.R + 15) / 16 * 128 > a.R * 9;
-  const bool start = CHORD && D > 96 && w8 <= grp::kLatWarps * 5 / 4;
+  const bool start = (!CHORD || D > 96) && w8 <= grp::kLatWarps * 5 / 4;
   if constexpr (P < 6)
-    if (D > 64 && w8 > grp::kLatWarps / 2 && (w8 <= grp::kLatWarps || waste || start || (a.R == 16 && D > 96)))
+    if (D > 64 && w8 > grp::kLatWarps / 2 && (w8 <= grp::kLatWarps || waste || start || (a.R <= 16 && D > 96)))
       return D <= 96 ? launch<32, 3, P, CHORD>(a, warps, st) : launch<32, 4, P, CHORD>(a, warps, st);
   if (w8 <= (D > 64 ? grp::kLatWarps / 2 : grp::kLatWarps))
     return D <= 32   ? launch<32, 1, P, CHORD, 1>(a, warps, st)
            : D <= 64 ? launch<32, 2, P, CHORD, 1>(a, warps, st)
            : D <= 96 ? launch<32, 3, P, CHORD, 1>(a, warps, st)
                      : launch<32, 4, P, CHORD, 1>(a, warps, st);
-  if (w8 <= grp::kOnePerWarp && D <= 64)
+  if (w8 <= (D > 16 ? grp::kOnePerWarp : 148LL * 32) && D <= 64)
     return D <= 32 ? launch<32, 1, P, CHORD>(a, warps, st) : launch<32, 2, P, CHORD>(a, warps, st);
   if (D <= 16 && (n <= grp::kMid16 || a.R < 16)) return launch<8, 2, P, CHORD>(a, warps, st);
   if (D <= 32 && D > 16 && (n <= grp::kMid32 || a.R < 16)) return launch<16, 2, P, CHORD>(a, warps, st);

@@ -5,7 +5,8 @@ Workload (one step = one pass of the hot path over one batch): 32 users x 32 ant
 i.i.d. Rayleigh channel uses with SNR 6-22 dB in 2 dB steps (round robin over the batch), one-stage dDI
 (K = 1, 128 spins) around the hard MMSE guess, 32 anneals per use, Arpeggio first-accept in fixed point at
 the reference's x32 budget (abl_far_32_0.1_0.1_0_rand_8: 32 sweeps x 2 passes, T 0.1, q 0, random start),
-then the distance readout: map (Gram + MMSE + quantise) -> anneal -> readout, three launches.
+then the distance readout: map (Gram + MMSE + quantise) -> anneal -> readout, three launches.  stdout gets one JSON
+line of under 2500 characters; stderr the same line with every block in full.
 
 metric: detections/s (whole job, all ranks), inputs resident in HBM (1.07 GB of channels per rank: larger
 than L2, no flush needed).  e2e: the same through Detector with pinned host buffers (H, y copied in, bits and
@@ -770,7 +771,7 @@ def _r(x, n=3):
 
 def summary(line):
     """The metric's other halves in a few hundred bytes, as the line's last key: warm vs plain (speed-up and the
-    paired BER-ratio intervals per SNR point), frame latency p50/p99, serving p99 per class at 1e5 frames/s."""
+    paired BER-ratio intervals per SNR point), frame latency p50/p99, serving p99 per class at 1e5 frames/s (full line)."""
     out = {'det_per_s': _r(line['value'], 4), 'e2e_det_per_s': _r(line['e2e']['value'], 4),
            'roofline_frac': _r(line['roofline']['frac']),
            'issue_frac': _r((line.get('roofline_issue') or {}).get('frac')),
@@ -810,6 +811,34 @@ def summary(line):
         out['mixed_det_per_s'] = _r(mx['value'])
         if mx.get('persistent'):
             out['mixed_persistent_det_per_s'] = _r(mx['persistent']['value'])
+    return out
+
+
+def short(line):
+    """The line for stdout: what identifies the run, its timings, the first roofline, the clocks and one number of each
+    other block, in under 2500 characters, so that the last few KB of a log hold it whole."""
+    keep = ('metric value unit n_gpus steps warmup ms_per_step higher_is_better scaling vs_baseline dtype data config e2e '
+            'stages_ms roofline gpu_launches clocks cpu_baseline').split()
+    out = {k: line[k] for k in keep if k in line}
+    out['e2e'] = {k: v for k, v in line['e2e'].items() if k not in ('path', 'steps')}
+    out['stages_ms'] = {k: _r(v, 5) for k, v in line['stages_ms'].items()}
+    out['roofline'] = {k: v for k, v in line['roofline'].items() if k not in ('ops_model', 'peak_source')}
+    if line.get('cpu_baseline'):
+        out['cpu_baseline'] = dict(line['cpu_baseline'], sample=line['cpu_baseline']['sample'].split(' (')[0])
+
+    def at(*path):
+        v = line
+        for k in path:
+            v = (v or {}).get(k)
+        return v
+    out['summary'] = {
+        'issue_frac': _r(at('roofline_issue', 'frac')),
+        'frame_us_p50_p99': [_r(at('latency', 'p50_us')), _r(at('latency', 'p99_us'))],
+        'warm_x_plain': {k: _r(at('warm_vs_plain', k, 'warm', 'speedup_vs_plain')) for k in ('x32', 'x64')},
+        'mdi_x16_per_s': _r(at('mdi_x16', 'value')), 'chord_x32_per_s': _r(at('extra', 'chord_x32', 'value')),
+        'mixed_per_s': _r(at('mixed', 'value')),
+        'serving_1e5_p99_ms': _r(max([v['p99_us'] / 1e3 for v in (
+            at('serving', 'rates', '1e+05 frames/s', 'per_class') or {}).values()], default=None))}
     return out
 
 
@@ -879,6 +908,9 @@ def main():
             import torch.distributed as dist
             dist.destroy_process_group()
     if line is not None:
+        if args.impl == 'ours':
+            print(json.dumps(line), file=sys.stderr, flush=True)  # every block in full
+            line = short(line)
         print(json.dumps(line), flush=True)
 
 

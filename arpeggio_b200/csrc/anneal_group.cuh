@@ -34,11 +34,9 @@
 // kMaxSched passes (every fixed-point problem of to_fixed, where |G|, |h| <= 4096) run with 32-bit energies and the
 // stored thresholds; the others run the same scan with 64-bit energies and one Philox block per pass (Wide).
 #pragma once
-#include <array>
 #include <climits>
 #include <mutex>
 #include <type_traits>
-#include <unordered_map>
 
 #include "arp_common.cuh"
 #include "arp_internal.h"
@@ -654,22 +652,32 @@ __global__ void __launch_bounds__(max_threads<LN, C>(), MB) k_anneal_grp(const D
 }
 
 // Per device: a kernel's resident blocks per SM at each block width (1, 2, 4, 8, 16 warps) for every shared-memory layout
-// it was launched with (one per staged schedule length: at most 130), and the dynamic shared memory it may use.  A launch
-// with a layout met before asks the runtime nothing.
+// it was launched with (one per staged schedule length), and the dynamic shared memory it may use.  A launch with a
+// layout met before asks the runtime nothing; nothing is allocated.
+constexpr int kLayouts = kMaxSched / 8 + 1;
 struct Widths {
   std::mutex mu;
   struct Dev {
-    size_t limit = 48 * 1024;
+    size_t limit = 0;  // 0: the 48 KB of every kernel
     int sms = 0;
-    std::unordered_map<size_t, std::array<int, 5>> nb;
+    struct {
+      bool known;
+      int8_t nb[5];
+    } layout[kLayouts] = {};
   } dev[kMaxDevices];
 };
-constexpr size_t kMaxDynamic = 226 * 1024;
+// The number of schedule length L's layout: its quads of sweeps, 0 where it is not staged.
+template <int P>
+inline int layout_of(int L) {
+  static_assert(P >= 2, "at least eight passes a quad");
+  return L <= kMaxSched ? (L + 4 * P - 1) / (4 * P) : 0;
+}
+constexpr size_t kMinDynamic = 48 * 1024, kMaxDynamic = 226 * 1024;
 
 // Launches kern for the A anneals per warp and blocks of at most WMAX warps it was compiled for; smem(W): its dynamic
-// shared memory with blocks of W warps, key: a number that differs where smem does.
+// shared memory with blocks of W warps, layout: a number below kLayouts that differs where smem does.
 template <int A, int WMAX, typename Kern, typename Smem>
-static cudaError_t launch_widths(Widths& wd, Kern kern, size_t key, Smem smem, const DDParams& a, int warps,
+static cudaError_t launch_widths(Widths& wd, Kern kern, int layout, Smem smem, const DDParams& a, int warps,
                                  cudaStream_t st) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -681,21 +689,23 @@ static cudaError_t launch_widths(Widths& wd, Kern kern, size_t key, Smem smem, c
     d.limit = bytes;
     return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   };
-  auto known = d.nb.find(key);
-  if (known == d.nb.end()) {
+  auto& known = d.layout[layout];
+  const int8_t* nb = known.nb;
+  if (!known.known) {
     if ((e = cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
     const size_t was = d.limit;
     if ((e = limit(kMaxDynamic)) != cudaSuccess) return e;
-    std::array<int, 5> n{};
     for (int i = 0; i < 5; ++i) {
+      int n = 0;
+      known.nb[i] = 0;
       if ((1 << i) > WMAX || smem(1 << i) > kMaxDynamic) continue;
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n[i], kern, 32 << i, smem(1 << i));
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, 32 << i, smem(1 << i));
       if (e != cudaSuccess) return e;
+      known.nb[i] = (int8_t)n;
     }
-    if ((e = limit(was)) != cudaSuccess) return e;
-    known = d.nb.emplace(key, n).first;
+    if ((e = limit(was > kMinDynamic ? was : kMinDynamic)) != cudaSuccess) return e;
+    known.known = true;
   }
-  const std::array<int, 5>& nb = known->second;
   const int sms = d.sms;
   // the width with the most resident warps per SM (ties: the wider block, which stages G fewer times per anneal),
   // or the caller's; no wider than the problem's anneals need
@@ -728,7 +738,7 @@ static cudaError_t launch_widths(Widths& wd, Kern kern, size_t key, Smem smem, c
       b.split = s;
     }
   }
-  if (smem(W) > d.limit && (e = limit(smem(W))) != cudaSuccess) return e;
+  if (smem(W) > (d.limit > kMinDynamic ? d.limit : kMinDynamic) && (e = limit(smem(W))) != cudaSuccess) return e;
   return launch_ex(kern, dim3((unsigned)((long long)a.B * b.split)), dim3(W * 32), smem(W), st, a.B <= kPdlMaxB, b);
 }
 
@@ -736,7 +746,7 @@ template <int LN, int C, int P, Rule RULE, int MB = min_blocks<LN, C>()>
 static cudaError_t launch(const DDParams& a, int warps, cudaStream_t st) {
   static Widths wd;
   return launch_widths<32 / LN, max_threads<LN, C>() / 32>(
-      wd, k_anneal_grp<LN, C, P, RULE, MB>, sched_bytes<P>(a.L),
+      wd, k_anneal_grp<LN, C, P, RULE, MB>, layout_of<P>(a.L),
       [&](int W) { return smem_bytes<LN, C, P, stored<LN, C, P, RULE, MB>()>(a.L, W); }, a, warps, st);
 }
 

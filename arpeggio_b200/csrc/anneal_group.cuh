@@ -45,7 +45,8 @@ namespace arp {
 namespace grp {
 
 constexpr int32_t kMaxG = 1 << 18, kMaxH = 1 << 28, kMaxT = 1 << 26;
-constexpr int kMaxSched = 1024;  // passes whose (4T, q + 2T - c) are staged in shared memory (8 KB)
+constexpr int kMaxSched = 8192;  // passes whose (4T, q + 2T - c) are staged in shared memory (64 KB)
+constexpr int kFineSched = 1024;  // above, the room is rounded up to this many passes
 constexpr int kMaxDevices = 64;
 
 enum Rule { kFirst, kWarm, kChord, kEngine };
@@ -467,7 +468,9 @@ __host__ __device__ constexpr size_t g_bytes() {
 }
 template <int P>
 __host__ __device__ inline size_t sched_bytes(int L) {
-  return L <= kMaxSched ? (size_t)((L + 4 * P - 1) / (4 * P) * 4 * P * 8 + 15) / 16 * 16 : 0;
+  constexpr int Q = 4 * P;  // a quad of sweeps
+  return L <= kFineSched ? (size_t)((L + Q - 1) / Q * Q * 8)
+         : L <= kMaxSched ? (size_t)((L + kFineSched - 1) / kFineSched * kFineSched + Q) * 8 : 0;
 }
 // Whether a kernel keeps stored thresholds.  The engine's numbers have none; and where six copies above 96 coordinates
 // fill the GPU (MB > 1) they are left out: 48 KB for eight warps beside 64 KB of G leave one block an SM instead of two,
@@ -654,7 +657,7 @@ __global__ void __launch_bounds__(max_threads<LN, C>(), MB) k_anneal_grp(const D
 // Per device: a kernel's resident blocks per SM at each block width (1, 2, 4, 8, 16 warps) for every shared-memory layout
 // it was launched with (one per staged schedule length), and the dynamic shared memory it may use.  A launch with a
 // layout met before asks the runtime nothing; nothing is allocated.
-constexpr int kLayouts = kMaxSched / 8 + 1;
+constexpr int kLayouts = kFineSched / 8 + kMaxSched / kFineSched + 1;
 struct Widths {
   std::mutex mu;
   struct Dev {
@@ -666,11 +669,12 @@ struct Widths {
     } layout[kLayouts] = {};
   } dev[kMaxDevices];
 };
-// The number of schedule length L's layout: its quads of sweeps, 0 where it is not staged.
+// The number of schedule length L's layout: its quads of sweeps or, of a long one, its thousands; 0 where it is not staged.
 template <int P>
 inline int layout_of(int L) {
   static_assert(P >= 2, "at least eight passes a quad");
-  return L <= kMaxSched ? (L + 4 * P - 1) / (4 * P) : 0;
+  return L <= kFineSched  ? (L + 4 * P - 1) / (4 * P)
+         : L <= kMaxSched ? kFineSched / 8 + (L + kFineSched - 1) / kFineSched : 0;
 }
 constexpr size_t kMinDynamic = 48 * 1024, kMaxDynamic = 226 * 1024;
 

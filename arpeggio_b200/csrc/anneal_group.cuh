@@ -102,7 +102,7 @@ __device__ __forceinline__ void load_row(uint32_t row, int ln, int32_t (&g)[C]) 
 }
 
 // The block's anneals of problem b: warp `wid` of block share bs takes A at a time.  Rb: anneals to run (<= R).
-template <int LN, int C, int P, Rule RULE, bool WIDE>
+template <int LN, int C, int P, Rule RULE, bool WIDE, bool SUM64 = WIDE>
 __device__ __forceinline__ void run(const DDParams& a, const PhiloxKeys& K, const int b, const int bs,
                                     const int32_t* Gs, const int2* sched, uint32_t* words, const uint8_t* s_perm,
                                     const uint32_t inst, const int Rb) {
@@ -121,7 +121,8 @@ __device__ __forceinline__ void run(const DDParams& a, const PhiloxKeys& K, cons
   constexpr bool SPREAD = LN == 32 && (WIDE || C <= 2);
   static_assert(P * C <= 32, "a lane's spins are one 32-bit word");
   static_assert(!ENG || WIDE, "the engine's numbers have no stored thresholds");
-  using ET = typename std::conditional<WIDE, long long, int32_t>::type;
+  using ET = typename std::conditional<WIDE, long long, int32_t>::type;   // a pass's sum
+  using DT = typename std::conditional<SUM64, long long, int32_t>::type;  // the running energy and the best
   const int D = a.D, L = a.L, R = a.R, split = a.split;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, W = blockDim.x >> 5;
   const int ln = lane & (LN - 1), grp = lane / LN;
@@ -227,7 +228,7 @@ __device__ __forceinline__ void run(const DDParams& a, const PhiloxKeys& K, cons
       for (int c = 0; c < C; ++c) w[c] = 0;
     }
     // energies in units of psi (a quarter of out_de); the engine's best register starts at 2^35 - 1
-    ET de = 0, best = ENG ? (ET)(1LL << 33) : WIDE ? (ET)(1LL << 60) : (ET)INT_MAX;
+    DT de = 0, best = ENG ? (DT)(1LL << 33) : sizeof(DT) == 8 ? (DT)(1LL << 60) : (DT)INT_MAX;
     uint32_t bdn = dn;
     int32_t flips = 0, lastflips = 0, n1 = 0;
     int k = 0;
@@ -472,14 +473,7 @@ __host__ __device__ inline size_t sched_bytes(int L) {
   return L <= kFineSched ? (size_t)((L + Q - 1) / Q * Q * 8)
          : L <= kMaxSched ? (size_t)((L + kFineSched - 1) / kFineSched * kFineSched + Q) * 8 : 0;
 }
-// Whether a kernel keeps stored thresholds.  The engine's numbers have none; and where six copies above 96 coordinates
-// fill the GPU (MB > 1) they are left out: 48 KB for eight warps beside 64 KB of G leave one block an SM instead of two,
-// and the energies of a fixed-point problem whose largest coefficient is in G are beyond 32 bits there (1500 60-user uses
-// of six copies, 8 anneals each: 2535 us with them, 1963 without; the kernel before the several-anneals ones 2304).
-template <int LN, int C, int P, Rule RULE, int MB>
-__host__ __device__ constexpr bool stored() {
-  return RULE != kEngine && !(LN == 32 && C == 4 && P == 6 && MB > 1);
-}
+// STORED: with the thresholds' room (the engine's numbers have none).
 template <int LN, int C, int P, bool STORED = true>
 inline size_t smem_bytes(int L, int W) {
   const size_t s = g_bytes<LN, C>() + sched_bytes<P>(L) + (STORED ? (size_t)W * P * C * 256 : 0);
@@ -490,7 +484,7 @@ inline size_t smem_bytes(int L, int W) {
 // One problem b of a block: G and the schedule staged in shared memory, then the block's anneals.  Called by the
 // per-launch kernel (one problem per block) and by the persistent mixed-size kernel (problems taken from a work
 // counter, one after another).
-template <int LN, int C, int P, Rule RULE, bool STORED = true>
+template <int LN, int C, int P, Rule RULE>
 __device__ __forceinline__ void problem(const DDParams& a, const PhiloxKeys& K, const int b, const int bs) {
   constexpr int DP = LN * C;
   constexpr bool CHORD = RULE == kChord || RULE == kEngine, WARM = RULE == kWarm;
@@ -622,14 +616,21 @@ __device__ __forceinline__ void problem(const DDParams& a, const PhiloxKeys& K, 
       }
     }
   }
-  if constexpr (!STORED) {
+  if constexpr (RULE == kEngine) {
     run<LN, C, P, RULE, true>(a, K, b, bs, Gs, sched, words, s_perm, inst, Rb);
   } else {
+    // What max |G| = 4096, a fixed-point problem's, puts beyond 32 bits: (2 P D + 2) 4096 P D >= 2^30 from P D = 362, two
+    // bits for the forms compiled (1: 32-bit sums, 2: 64-bit ones of 32-bit passes).  Six copies below 61 coordinates lose
+    // 4 % with the wider sums (2000 30-user uses by Chord 829 -> 862 us), at 64 they gain (1409 -> 949; 64-bit throughout before).
+    constexpr int SUMS = LN * C * P <= 361 ? 1 : (P == 6 && DP == 64) || (P == 4 && DP == 96) ? 3 : 2;
     // |psi| <= |h| + (2 P D + 2) max |G| at any state; a pass adds at most D of them and the energy of any state
-    // stays within D P / 2 of them, so below 2^30 / (D P) every sum fits 32 bits
+    // stays within D P / 2 of them, so below 2^30 / (D P) every sum fits 32 bits, below 2^30 / D those of a pass
     const long long psi = (long long)s_mh + (2LL * P * D + 2) * s_mg;
-    if (psi * D * P < (1LL << 30) && !s_wt && L <= kMaxSched)
+    const bool pass = psi * D < (1LL << 30) && !s_wt && L <= kMaxSched;
+    if ((SUMS & 1) && pass && psi * D * P < (1LL << 30))
       run<LN, C, P, RULE, false>(a, K, b, bs, Gs, sched, words, s_perm, inst, Rb);
+    else if ((SUMS & 2) && pass)
+      run<LN, C, P, RULE, false, true>(a, K, b, bs, Gs, sched, words, s_perm, inst, Rb);
     else
       run<LN, C, P, RULE, true>(a, K, b, bs, Gs, sched, words, s_perm, inst, Rb);
   }
@@ -651,7 +652,7 @@ __global__ void __launch_bounds__(max_threads<LN, C>(), MB) k_anneal_grp(const D
   const int split = a.split, b = blockIdx.x / split, bs = blockIdx.x - b * split;
   pdl_trigger();
   pdl_wait();
-  problem<LN, C, P, RULE, stored<LN, C, P, RULE, MB>()>(a, *reinterpret_cast<const PhiloxKeys*>(a.rk0), b, bs);
+  problem<LN, C, P, RULE>(a, *reinterpret_cast<const PhiloxKeys*>(a.rk0), b, bs);
 }
 
 // Per device: a kernel's resident blocks per SM at each block width (1, 2, 4, 8, 16 warps) for every shared-memory layout
@@ -751,7 +752,7 @@ static cudaError_t launch(const DDParams& a, int warps, cudaStream_t st) {
   static Widths wd;
   return launch_widths<32 / LN, max_threads<LN, C>() / 32>(
       wd, k_anneal_grp<LN, C, P, RULE, MB>, layout_of<P>(a.L),
-      [&](int W) { return smem_bytes<LN, C, P, stored<LN, C, P, RULE, MB>()>(a.L, W); }, a, warps, st);
+      [&](int W) { return smem_bytes<LN, C, P, RULE != kEngine>(a.L, W); }, a, warps, st);
 }
 
 // How many anneals share a warp is a matter of how many there are: A per warp need A times as many to fill the GPU.
@@ -787,8 +788,11 @@ static cudaError_t dispatch(const DDParams& a, int warps, cudaStream_t st) {
   // bound for blocks of 16 warps, keep two of them an SM, one per warp four (3000 53-user uses, 16 anneals, easy ones 4:
   // 2667 -> 2420 us; 64-user ones 2705 -> 2440).  Up to 96 coordinates two per warp stay ahead (1790 against 1830).
   const bool counted = RULE == kWarm && a.ra && D > 96;
+  // Four copies above 96 coordinates, up to 16 anneals: eight two-per-warp warps' thresholds (64 KB beside as much of G)
+  // leave one block an SM, one per warp two (1000 64-user uses of 16: first accept 621 -> 479 us, Chord 1120 -> 856).
+  const bool room = P == 4 && D > 96 && a.R <= 16;
   if constexpr (RULE != kEngine && P < 6)
-    if (D > 64 && w8 > kLatWarps / 2 && (w8 <= kLatWarps || ragged || waste || start || counted))
+    if (D > 64 && w8 > kLatWarps / 2 && (w8 <= kLatWarps || ragged || waste || start || counted || room))
       return D <= 96 ? launch<32, 3, P, RULE>(a, warps, st) : launch<32, 4, P, RULE>(a, warps, st);
   if (RULE != kEngine && w8 <= (D > 64 ? kLatWarps / 2 : kLatWarps))
     return D <= 32   ? launch<32, 1, P, RULE, 1>(a, warps, st)

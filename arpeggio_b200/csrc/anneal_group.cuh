@@ -118,7 +118,7 @@ __device__ __forceinline__ void run(const DDParams& a, const PhiloxKeys& K, cons
   // 64 bits (five steps of two shuffles), a flip's psi goes to every lane by a shuffle beside its factor's and no
   // reduction stands between one pass and the next.  64 sweeps, chain of map, anneal and readout, with the reduction
   // against without: one 32-user frame 86.9 -> 81.4 us, one 8-user frame 37.1 -> 33.9, 40 9-user frames 58.9 -> 53.7.
-  constexpr bool SPREAD = LN == 32 && (WIDE || C <= 2);
+  constexpr bool SPREAD = LN == 32 && (CHORD ? !WIDE && C <= 2 && P == 2 : WIDE || C <= 2);
   static_assert(P * C <= 32, "a lane's spins are one 32-bit word");
   static_assert(!ENG || WIDE, "the engine's numbers have no stored thresholds");
   using ET = typename std::conditional<WIDE, long long, int32_t>::type;   // a pass's sum

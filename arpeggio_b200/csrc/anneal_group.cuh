@@ -766,6 +766,12 @@ static cudaError_t launch(const DDParams& a, int warps, cudaStream_t st) {
 // per warp keeps its lead into a short second wave (37 warps a SM for 32): 76 and 83 14-user uses of 64 anneals in the
 // chain of map, anneal and readout 74 -> 67 and 79 -> 78 us, 120 21-user uses of 33 104 -> 93.
 constexpr long long kLatWarps = 148LL * 16, kOnePerWarp = 148LL * 37;
+// (by registers: 12 a SM with two coordinates a lane and four or six copies, 8 above 64 coordinates; 120 60-user uses of
+// four copies, 16 anneals: 72 -> 57 us with the bound kernel; the kernel before 56)
+template <int P>
+inline long long lat_warps(int D) {
+  return D > 64 ? kLatWarps / 2 : P > 2 && D > 32 ? kLatWarps * 3 / 4 : kLatWarps;
+}
 constexpr long long kMid16 = 30000, kMid32 = 10000, kMid64 = 148LL * 32 * 8;
 
 // The mapping (LN lanes per anneal, C coordinates per lane) for D coordinates.  P = 6 keeps four coordinates a lane
@@ -795,7 +801,7 @@ static cudaError_t dispatch(const DDParams& a, int warps, cudaStream_t st) {
   if constexpr (RULE != kEngine && P < 6)
     if (D > 64 && w8 > kLatWarps / 2 && (w8 <= kLatWarps || ragged || waste || start || counted || room))
       return D <= 96 ? launch<32, 3, P, RULE>(a, warps, st) : launch<32, 4, P, RULE>(a, warps, st);
-  if (RULE != kEngine && w8 <= (D > 64 ? kLatWarps / 2 : kLatWarps))
+  if (RULE != kEngine && w8 <= lat_warps<P>(D))
     return D <= 32   ? launch<32, 1, P, RULE, 1>(a, warps, st)
            : D <= 64 ? launch<32, 2, P, RULE, 1>(a, warps, st)
            : D <= 96 ? launch<32, 3, P, RULE, 1>(a, warps, st)

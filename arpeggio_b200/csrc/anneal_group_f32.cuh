@@ -292,7 +292,7 @@ static cudaError_t dispatch(const DDParams& a, int warps, cudaStream_t st) {
   if constexpr (P < 6)
     if (D > 64 && w8 > grp::kLatWarps / 2 && (w8 <= grp::kLatWarps || waste || start || (a.R <= 16 && D > 96)))
       return D <= 96 ? launch<32, 3, P, CHORD>(a, warps, st) : launch<32, 4, P, CHORD>(a, warps, st);
-  if (w8 <= (D > 64 ? grp::kLatWarps / 2 : grp::kLatWarps))
+  if (w8 <= grp::lat_warps<P>(D))
     return D <= 32   ? launch<32, 1, P, CHORD, 1>(a, warps, st)
            : D <= 64 ? launch<32, 2, P, CHORD, 1>(a, warps, st)
            : D <= 96 ? launch<32, 3, P, CHORD, 1>(a, warps, st)

@@ -806,7 +806,7 @@ static cudaError_t dispatch(const DDParams& a, int warps, cudaStream_t st) {
            : D <= 64 ? launch<32, 2, P, RULE, 1>(a, warps, st)
            : D <= 96 ? launch<32, 3, P, RULE, 1>(a, warps, st)
                      : launch<32, 4, P, RULE, 1>(a, warps, st);
-  if (RULE != kEngine && w8 <= (D > 16 ? kOnePerWarp : 148LL * 32) && D <= 64)
+  if (w8 <= (D > 16 ? kOnePerWarp : 148LL * 32) && D <= 64)
     return D <= 32 ? launch<32, 1, P, RULE>(a, warps, st) : launch<32, 2, P, RULE>(a, warps, st);
   // few anneals a use leave a wide block's warps without work: the half mapping below 16
   if (D <= 16 && (n <= kMid16 || a.R < 16)) return launch<8, 2, P, RULE>(a, warps, st);

@@ -1,5 +1,5 @@
-"""Schedules on both sides of what is staged and running energies beyond 32 bits with stored thresholds (four copies above 90
-coordinates, six above 60), bit for bit against the oracle."""
+"""Schedules on both sides of what is staged, running energies beyond 32 bits with stored thresholds (four copies above 90
+coordinates, six above 60), and the engine's numbers on its small and large mappings, bit for bit against the oracle."""
 import numpy as np
 import pytest
 import torch
@@ -50,3 +50,20 @@ def test_energies_beyond_32_bits(D, P, B, R, policy):
     h[:, ::3] *= -1
     de = _same(D, P, B, R, T, 60, policy, G, h)
     assert P < 6 or np.abs(de[::2]).max() > 4 * 2 ** 31
+
+
+@pytest.mark.parametrize('D,P', [(8, 2), (16, 4), (17, 2), (32, 6), (33, 4), (64, 2), (64, 6), (96, 2), (128, 4)])
+@pytest.mark.parametrize('B,R', [(3, 5), (90, 9), (700, 9)])
+def test_engine_numbers(D, P, B, R):
+    from arpeggio_b200 import arpeggiofx
+    from test_gpu_anneal_group import _problems
+    G, h = _problems(D, B, 2)
+    T, c = np.array([900, 700, 500, 410, 300]), np.array([10, -30, 0, 20, 5])
+    inst, key = np.arange(B, dtype=np.int64) + 9, 0x4242 + (0x99 << 32)
+    ref = O.anneal_chord_hw(G, h, P, R, T, c, 60, inst, key, nthreads=NTH)
+    dev = lambda x: torch.from_numpy(np.ascontiguousarray(x, dtype=np.int32)).cuda()
+    s, de, st, status = arpeggiofx.anneal_engine(dev(G), dev(h), P, R, dev(T), 60, dev(inst), key, dev(c))
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    for got, want in zip((s, de, st), ref):
+        assert np.array_equal(got.cpu().numpy(), want)

@@ -376,9 +376,11 @@ __global__ void __launch_bounds__(32 * kSoftWarps) k_traj_soft(const SoftParams 
 template <int LN, int CD, bool QAM>
 static cudaError_t launch_soft(const SoftParams& a, cudaStream_t st) {
   using M = SoftMap<LN, CD, QAM>;
-  // up to 64 spins the chains' warps stage J alone: more warps would hold registers that other blocks' chains need
-  // (1400 uses of 64 spins, one chain each: 1345 us with one warp, 1547 with two)
-  const int W = min(kSoftWarps, (a.R + M::A - 1) / M::A), stage = a.N <= 64 ? 1 : a.N <= 96 ? 4 : kSoftWarps;
+  // up to 64 spins, and up to 96 where the problems fill the GPU, the chains' warps stage J alone: more warps would hold
+  // registers that other blocks' chains need (one chain each: 1400 uses of 64 spins 1345 us with one warp, 1547 with two;
+  // 3000 of 72, with their LLRs, 10.4 ms with one, 11.8 with two, 12.7 with four; 3000 of 128 21.7 with four, 23.7 with two,
+  // 27.8 with eight)
+  const int W = min(kSoftWarps, (a.R + M::A - 1) / M::A), stage = a.N <= 64 || (a.N <= 96 && a.B > 296) ? 1 : 4;
   const size_t smem = 4 * ((size_t)a.N * M::DP + (size_t)W * 4 * M::C * 32 + (size_t)W * 2 * CD * M::NB * LN +
                            kSoftWarps * 3 + (size_t)W * LN);
   if (smem > 48 * 1024) {

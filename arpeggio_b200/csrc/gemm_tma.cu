@@ -250,6 +250,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   } else if (warp == 1) {
     if (lane == 0) {
       // ---- MMA issue
+      const int whole = p.K >> 6;  // k tiles without zeros past K
       int slot = 0, it = 0;
       uint32_t ph = 0;
       for (int item = blockIdx.x; item < wk.items && !s_abort; item += gridDim.x, ++it) {
@@ -272,12 +273,17 @@ __global__ void __launch_bounds__(kThreads, 1)
           umma::tc_after_sync();
           const uint32_t sa = ring + (uint32_t)slot * SBYTES;
           const uint32_t sb = ring + (uint32_t)(keep_b ? kt : slot) * SBYTES + kABytes;
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk) {
-            if (kt * 64 + kk * 16 >= p.K) break;  // past K the tiles hold zeros
+          auto mma = [&](int kk) {
             const uint64_t ad = AMN ? umma::sdesc_sw128(sa + kk * 2048, 8192, 1024) : umma::sdesc_sw128(sa + kk * 32, 16, 1024);
             const uint64_t bd = BMN ? umma::sdesc_sw128(sb + kk * 2048, 8192, 1024) : umma::sdesc_sw128(sb + kk * 32, 16, 1024);
             umma::mma(acc, ad, bd, IDESC, (kt > kt0 || kk > 0) ? 1u : 0u);
+          };
+          if (kt < whole) {
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) mma(kk);
+          } else {  // past K the tiles hold zeros
+#pragma unroll 1
+            for (int kk = 0; kt * 64 + kk * 16 < p.K; ++kk) mma(kk);
           }
           umma::commit(&empty[slot]);
           if (++slot == S) {

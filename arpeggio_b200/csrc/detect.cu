@@ -535,17 +535,17 @@ __global__ void __launch_bounds__(MapShape<TB, RB_, U_>::NT, MapShape<TB, RB_, U
       zp[i] = row_dot<TB>(ar, gj);
       mp[i] = row_dot<TB>(ar, qj);
     }
-    if (tx == 0) {  // to shared memory (row buffer: the last step's readers of its halves are behind a barrier)
+    if (tx == 0) {  // to shared memory (mu to the half of ck that the last step, an odd one, does not read)
 #pragma unroll
       for (int i = 0; i < RB; ++i) {
         xv[ty * RB + i] = zp[i];
-        ck[Dp + ty * RB + i] = mp[i];
+        ck[ty * RB + i] = mp[i];
       }
     }
     __syncthreads();
     if (ut < Dp) {
       const float z = xv[ut];
-      const float zu = ut < D ? __fdiv_rn(z, ck[Dp + ut]) : 0.0f;
+      const float zu = ut < D ? __fdiv_rn(z, ck[ut]) : 0.0f;
       const float lv = ut < D ? nearest_level(zu, a.M) : 0.0f;
       if (on && ut < D) {
         a.xq[(size_t)b * D + ut] = (int8_t)lv;

@@ -212,9 +212,10 @@ __device__ __forceinline__ void run(const DDParams& a, const PhiloxKeys& K, cons
 #pragma unroll
     for (int c = 0; c < C; ++c) {
       // every spin sum of the slot 0 in every anneal of the warp ('bal' with two copies; most slots of a warm start):
-      // nothing to add (3000 64-user uses from 'bal', 33 anneals x 24 sweeps, 3985 -> 3800 us); not by Chord, whose passes
-      // are many and lose more to it (700 18-user uses of six copies 334 -> 318 us, a 32-user use with T = 5 115 -> 108)
-      if (!CHORD && !__any_sync(ARP_FULL, m2[c] != 0)) continue;
+      // nothing to add (3000 64-user uses from 'bal', 33 anneals x 24 sweeps, 3985 -> 3800 us); not asked of random starts
+      // (65536 32-user uses, 32 anneals: 22.75 ms asking, 22.36 not), nor by Chord, whose passes are many and lose more to
+      // the code it makes (700 18-user uses of six copies 334 -> 318 us, a 32-user use with T = 5 115 -> 108)
+      if (!CHORD && (WARM || a.start != 0) && !__any_sync(ARP_FULL, m2[c] != 0)) continue;
 #pragma unroll(LN == 32 ? 4 : 2)
       for (int i = 0; i < (LN == 32 ? min(LN, D - c * LN) : LN); ++i) {  // coordinate c LN + i, on lane LN - 1 - i
         const int32_t m = __shfl_sync(ARP_FULL, m2[c], LN - 1 - i, LN);

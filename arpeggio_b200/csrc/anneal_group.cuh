@@ -13,7 +13,7 @@
 // in a round (it runs while any group has one), which bounds how far this goes.  Measured per 8192 32-user uses
 // (32 anneals x 64 passes): one anneal per warp with two coordinates per lane 4.2 ms (the previous kernel; 3.7 ms in
 // this form), two anneals with four 3.2 ms, four anneals with eight 2.9 ms; in instructions per anneal 14.6 k, 12.7 k
-// (this form), 10.6 k, 9.5 k.  The issue slots bound it (80 % busy at 32 resident warps per SM).
+// (this form), 10.6 k, 9.76 k.  The issue slots bound it (79 % busy at 32 resident warps per SM).
 //
 // Margins.  For its copy's spin s a lane adds x = s ? ~e : e to w on entering a slot, with e = kappa - 2 G_jj - 1 and
 // kappa = ceil(u 4T / 2^32) - q - 2T (+ c): then z = (w + x) XOR (s up ? 0 : -1) equals psi - kappa, psi = s w + 2 G_jj,
@@ -30,9 +30,10 @@
 // x two copies x four sweeps would be 64 registers a lane as words), written and read by the same lane.
 //
 // Ranges.  |G| <= 2^18, |h| <= 2^28, |T|, |q|, |c| <= 2^26 keep every field, margin and threshold inside int32
-// (ARP_ERR_RANGE otherwise).  Problems whose energies fit 32 bits and whose schedule has 0 <= T < 2^14 and at most
-// kMaxSched passes (every fixed-point problem of to_fixed, where |G|, |h| <= 4096) run with 32-bit energies and the
-// stored thresholds; the others run the same scan with 64-bit energies and one Philox block per pass (Wide).
+// (ARP_ERR_RANGE otherwise).  Problems whose pass sums fit 32 bits (every fixed-point problem of to_fixed, where |G|,
+// |h| <= 4096) and whose schedule has 0 <= T < 2^14 and at most kMaxSched passes run with the stored thresholds, and with a
+// 32-bit running energy where that fits too; the others run the same scan with 64-bit energies and one Philox block per
+// pass (WIDE).
 #pragma once
 #include <climits>
 #include <mutex>
@@ -117,7 +118,9 @@ __device__ __forceinline__ void run(const DDParams& a, const PhiloxKeys& K, cons
   // One anneal per warp: where its latency is what counts (up to two coordinates a lane), or the reduction would be of
   // 64 bits (five steps of two shuffles), a flip's psi goes to every lane by a shuffle beside its factor's and no
   // reduction stands between one pass and the next.  64 sweeps, chain of map, anneal and readout, with the reduction
-  // against without: one 32-user frame 86.9 -> 81.4 us, one 8-user frame 37.1 -> 33.9, 40 9-user frames 58.9 -> 53.7.
+  // against without: one 32-user frame 86.9 -> 81.4 us, one 8-user frame 37.1 -> 33.9, 40 9-user frames 58.9 -> 53.7.  By
+  // Chord only with two copies and 32 bits: passes with many flips pay per flip (120 32-user uses of four copies, 16
+  // anneals, 128 passes: 139 us with the reduction, 164 without).
   constexpr bool SPREAD = LN == 32 && (CHORD ? !WIDE && C <= 2 && P == 2 : WIDE || C <= 2);
   static_assert(P * C <= 32, "a lane's spins are one 32-bit word");
   static_assert(!ENG || WIDE, "the engine's numbers have no stored thresholds");

@@ -21,7 +21,8 @@ struct MixedArgs {
   DDParams cls[kMaxMixed];
 };
 
-// The mapping of each slot count's group, as the per-class dispatch picks it for large batches.
+// The mapping of each slot count's group: one that holds its largest coordinate count (the per-class dispatch picks
+// narrower ones for large batches up to 16 coordinates and from 33 to 48).
 template <int NS>
 struct MixedMap {
   static constexpr int LN = NS <= 2 ? 8 : 16, C = NS == 1 ? 4 : NS == 3 ? 6 : 8;

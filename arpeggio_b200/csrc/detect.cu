@@ -124,7 +124,7 @@ __device__ __forceinline__ float row_dot(const float (&x)[TB], const float (&y)[
 // padded diagonal of A is 1, so the inverse's D x D block is unchanged.  A block holds U uses (U Dp = 64 rows of one
 // MMA for Dp <= 64).  What bounds the map is issue slots and the elimination's latency (one barrier a step), so:
 //   tall tiles: an elimination step loads RB + TB values and forms RB factors for RB TB multiply-adds.  8 x 4 on
-//     128 threads (37 k instructions per 32-user use, then the code's own fetches) against 4 x 4 on 256 (45 k, the
+//     128 threads (34.7 k instructions per 32-user use, then the code's own fetches) against 4 x 4 on 256 (47.9 k, the
 //     previous kernel): 16384 32-user uses 0.90 -> 0.76 ms; a batch of 444 uses or fewer keeps 4 x 4;
 //   several uses per block where D is small, which share the barriers and the MMAs: 49999 8-user uses 1.04 -> 0.35 ms,
 //     16384 16-user ones 0.42 -> 0.27;

@@ -44,7 +44,7 @@ struct Partials {
 };
 
 enum { EPI_F32 = 0, EPI_F32_ACC = 1, EPI_BIAS_RELU_BF16 = 2, EPI_BIAS_F32 = 3, EPI_MASK_BF16 = 4 };
-// Internal: split z of a split-K product stores its partial tile at C + z M ldc (summed afterwards in split order).
+// Internal: split z of a split-K product stores its partial tile at C + z M ldc (summed afterwards in a fixed order).
 constexpr int EPI_F32_PART = 5;
 
 template <int CW>
@@ -100,11 +100,12 @@ __device__ __forceinline__ void epilogue(const GemmParams& p, int row, int n, co
   }
 }
 
-// C (M x N, leading dimension ldc) += the split-K partials ws[0 .. splits-1] (dense M x N each), summed in split
-// order on the stream (warm.cu).
+// C (M x N, leading dimension ldc) += the split-K partials ws[0 .. splits-1] (dense M x N each), summed in a
+// fixed order on the stream (warm.cu).
 cudaError_t sum_splits(const float* ws, int splits, int M, int N, float* C, int ldc, cudaStream_t st);
 
-// The TMA-fed, warp-specialised kernel (gemm_tma.cu) for products with M >= 128, N >= 64 and K >= 64;
+// The TMA-fed, warp-specialised kernel (gemm_tma.cu) for products with M >= 128 (accumulating ones also N >= 64
+// and K >= 64);
 // cudaErrorNotSupported when the driver's tensor-map encoder is unavailable or refuses the operands.
 bool gemm_tma_fits(const GemmParams& p);
 cudaError_t gemm_tma(const GemmParams& p, bool a_mn, bool b_mn, cudaStream_t st);

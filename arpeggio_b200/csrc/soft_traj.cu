@@ -19,11 +19,12 @@
 // CD + cc (the LSB spin D + j), so slots and lanes ascend with the spin index and a coordinate's two spins share a
 // lane.  A round commits one flip of every chain of the warp, and a slot's rounds are counted once (the largest number
 // of flips among the chains) instead of voted on.  What bounds it is the rows of J: a flip reads one, two wavefronts
-// of shared memory at 64 spins, and they keep its pipe 71 % busy (issue slots 60 %; 1990 instructions per step of four
-// chains, 1826 per step of one before).  4096 16-user uses, 16 chains x 256 steps: 32.5 -> 11.6 ms.
+// of shared memory at 64 spins, and they keep its pipe 81 % busy (issue slots 67 %; 2018 instructions per step of four
+// chains, 1826 per step of one before).  4096 16-user uses, 16 chains x 256 steps: 32.5 -> 11.1 ms.
 // With few chains a problem's blocks are what is resident, so J takes a row per spin and columns to the next multiple of
-// LN only (36 KB at 96 spins), and where it is large more warps than the chains need help to stage it: 1400 24-user
-// uses of one 64-step chain 2796 us with 64 KB rounded up to whole slots and one warp, 1927 now; of five 3171 and 2280.
+// LN only (36 KB at 96 spins), and where it is large, or the problems few, four warps stage it though fewer run chains:
+// 1400 24-user uses of one 64-step chain 2796 us with 64 KB rounded up to whole slots, 1927 with the rows (and four warps;
+// one warp is as fast there, see launch_soft); of five 3171 and 2280.
 // The reference draws its chains' start and tests from torch.rand; this sampler draws them from Philox counters of
 // its own (start: word 0 of (2^32 - 1, i, r, inst), spin +1 iff >= 2^31), so its trajectories are its own while the
 // rule, the visited-state bookkeeping and the LLR formation are the reference's.

@@ -67,8 +67,7 @@ def detect(H, y, N0, M, seed, pick, Rmax=None, stages=None, policy='arpeggio', p
     ann = np.zeros(B)
     cnt = counters if counters is not None else {}
     # the counters stay on the device until the walk is over: per K the sum over the anneals of (flips, tests) and n1,
-    # and the anneals counted here (reading them group by group drained the queue each time: 45 against 39 ms for
-    # 8192 16-user 16-QAM uses)
+    # and the anneals counted here (reading them group by group drained the queue each time)
     dev_cnt, host_cnt = {}, {}
     seed_base = (seed * 0x9E3779B97F4A7C15) & M64
     calls = 0

@@ -727,8 +727,11 @@ static cudaError_t launch_widths(Widths& wd, Kern kern, int layout, Smem smem, c
   while (wi > 0 && (1 << (wi - 1)) * A >= a.R) --wi;
   // one anneal per warp, every block resident at once: blocks of eight warps, or of four where those leave fewer warps on
   // the fullest SM (one 32-user frame: 44 us against 46 with eight; 37 26-user frames, 33 anneals a use, in the chain
-  // of map, anneal and readout: 70 against 75; 64 32-user frames: 69 against 63 with eight)
-  if (A == 1 && warps <= 0 && (wi == 2 || wi == 3) && a.R > 4) {
+  // of map, anneal and readout: 70 against 75; 64 32-user frames: 69 against 63 with eight); above 16 warps a SM not in a
+  // programmatic launch, whose blocks wait beside the map's: 60 17-user uses of 33 in that chain 63.8 us with four, 56.7 with
+  // eight (the kernel before 53.6), 64 32-user uses of 64 82.1 and 74.0 (104.1)
+  const bool beside = a.B <= kPdlMaxB && a.B * (long long)((a.R + 7) / 8 * 8) > 16LL * sms;
+  if (A == 1 && warps <= 0 && (wi == 2 || wi == 3) && a.R > 4 && !beside) {
     const auto fullest = [&](int W) { return (a.B * (long long)((a.R + W - 1) / W) + sms - 1) / sms; };
     if (fullest(8) <= nb[3] && fullest(4) <= nb[2]) wi = 4 * fullest(4) < 8 * fullest(8) ? 2 : 3;
   }
